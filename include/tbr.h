@@ -109,7 +109,7 @@ typedef struct tbr_ext_options {
     int32_t points_per_iter;      /* scoring tile: 0 = default, 2 or 4 points per inner step of the
                                      FP32 kernel (an FP32 field alone selects the FP32 kernel, the
                                      other field then 4 / 2), 128 = tensor-core scoring (tcgen05 MMA
-                                     over 128-point tiles, 32 hypotheses per block; the default) */
+                                     over 64-point tiles, 128 hypotheses per block; the default) */
 } tbr_ext_options;
 
 /* Results of one estimate. The reference returns RansacStats_cuda unfilled except
@@ -293,7 +293,7 @@ tbr_status tbr_batch_profile(tbr_batch *b, tbr_kernel_profile *out, int32_t max,
  * `repeats` times under each candidate shape -- FP32: hypotheses per warp block
  * (32 x hyp_per_thread: 64, 128, 192, 256), points per iteration (2, 4) and points
  * per work-item tile (0 = sized from the step's work, 256, 512, 1024, 2048);
- * tensor cores: points_per_iter = 128 (32 hypotheses per block, reported as
+ * tensor cores: points_per_iter = 128 (128 hypotheses per block, reported as
  * hyp_per_thread = 1) with tiles 0 and 8192; 32 candidates in all --
  * and keeps the fastest for later tbr_batch_run calls. The shape changes only
  * the order of FP32 partial sums inside the filter; every candidate within the

@@ -111,7 +111,7 @@ struct RunOptions {
     double trials_mult = 3.0;
     int skip_refine = 0;
     int quirk = 0;
-    // Scoring shape: hr = 1 is the tensor-core kernel (32 hypotheses per block,
+    // Scoring shape: hr = 1 is the tensor-core kernel (128 hypotheses per block,
     // pp = kTcPP), the default; hr = 2, 4, 6, 8 with pp = 2 or 4 the FP32 kernels.
     int hr = 1;
     int pp = kTcPP;
@@ -481,7 +481,7 @@ class Engine {
     // Scoring kernel variant: HR hypotheses per lane = 2*HP, PP points per iteration.
     void launch_score(const Pools &Q, int hr, int pp, cudaStream_t st) {
         const int threads = kScoreWarps * 32;
-        if (hr == 1) k_score_tc<<<4 * num_sms, kTcThreads, kTcSmem, st>>>(Q);  // (pp == kTcPP)
+        if (hr == 1) k_score_tc<<<kTcCtas * num_sms, kTcThreads, kTcSmem, st>>>(Q);  // (pp == kTcPP)
         else if (hr == 2) k_score<1, 4><<<score_grid[0], threads, 0, st>>>(Q);
         else if (hr == 8) k_score<4, 2><<<score_grid[3], threads, 0, st>>>(Q);
         else if (hr == 6 && pp == 4) k_score<3, 4><<<score_grid[5], threads, 0, st>>>(Q);
@@ -2105,7 +2105,7 @@ tbr_status tbr_batch_autotune(tbr_batch *b, int32_t repeats, tbr_tune_entry *ent
     struct Shape {
         int hr, pp;
     };
-    // Hypotheses per block x point tile per work item: 32 (the tensor-core
+    // Hypotheses per block x point tile per work item: 128 (the tensor-core
     // kernel) and 64 / 128 / 192 / 256 (the compiled FP32 variants, 2 / 4 / 6 / 8
     // per lane, with 2 or 4 points per inner step) x tiles of 128, 256 and 512
     // points, plus tiles sized from the step's work (0) and longer ones.
@@ -2125,6 +2125,9 @@ tbr_status tbr_batch_autotune(tbr_batch *b, int32_t repeats, tbr_tune_entry *ent
     TBR_CUDA(cudaEventCreate(&t1));
     auto apply = [&](int hr, int pp, int chunk, cudaGraph_t *g, cudaGraphExec_t *x) -> bool {
         k_set_shape<<<(n + 127) / 128, 128, 0, E.stream>>>(b->d_init, n, hr, chunk);
+        // The staging blocks' layout follows the shape's kernel (k_prep_pack).
+        k_reset_frames<<<n, 128, 0, E.stream>>>(b->Q, b->d_init);
+        k_prep_pack<<<dim3(Engine::prep_bx(*std::max_element(b->ns.begin(), b->ns.end())), n), 256, 0, E.stream>>>(b->Q);
         if (cudaGetLastError() != cudaSuccess) return false;
         E.pp = pp;
         return E.build_loop_graph(b->Q, n, hr, b->d_init, g, x);

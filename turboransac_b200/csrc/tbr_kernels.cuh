@@ -36,6 +36,8 @@ constexpr int kMaxScoreChunks = 64;               // FP32 scoring point chunks p
 constexpr int kMaxActive = 1024;                  // frames advanced by one step
 constexpr uint32_t kMaxPolls = 1u << 26;          // bounded mbarrier waits (~seconds)
 constexpr int kScoreWarps = 4;                    // warps per scoring CTA
+constexpr int kTcCtas = 2;                          // ... and its CTAs per SM (tensor memory)
+constexpr int kTcHyp = 128;                       // tensor-core scoring: hypotheses per item (MMA M), a thread each
 constexpr int kLMThreads = 256;       // per CTA of a cluster LM (two CTAs per SM)
 constexpr int kLMSmallThreads = 384;  // one CTA per frame: 12 warps, no register spills
 
@@ -252,6 +254,11 @@ __device__ __forceinline__ int find_segment(const int64_t *prefix, int n, int64_
     return lo;
 }
 
+// Rounded to nearest TF32 (11 significant bits).
+__device__ __forceinline__ float tf32_rn(float x) {
+    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
+}
+
 __device__ __forceinline__ void flag_error(const Pools &P, unsigned long long bits) {
     atomicOr(&P.counters[kCError], bits);
 }
@@ -289,9 +296,30 @@ __global__ void k_prep_bounds(Pools P) {
     }
 }
 
-// Normalized coordinates (Camera_cuda::unproject, camera.cuh:51-62) and the FP32
-// staging blocks: centred world points and -x/tau, -y/tau, each duplicated so
+// The FP32 filter's view of a point: the centred world point and -x/tau, -y/tau.
+// Non-finite points (never an FP64 inlier) and points beyond 2^80 become outliers
+// for every pose.
+__device__ __forceinline__ void stage_point(const double *X, double xn, double yn, const double *c, double itau,
+                                            float (&v)[5]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = (float)(X[k] - c[k]);
+    v[3] = (float)(-xn * itau);
+    v[4] = (float)(-yn * itau);
+    bool finite = true;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) finite = finite && fabsf(v[k]) <= 0x1p80f;
+    if (!finite) {
+        v[0] = v[1] = v[2] = 0.0f;
+        v[3] = v[4] = 0x1p100f;
+    }
+}
+
+// Normalized coordinates (Camera_cuda::unproject, camera.cuh:51-62) and the
+// staging blocks of the frame's scoring shape. FP32 kernels: each value twice, so
 // that one 64-bit lane pair feeds both halves of a packed FP32x2 instruction.
+// Tensor-core kernel: two 32-point B operands ([hi xyz, 1 | lo xyz, 0] rows in
+// 8-row x 16-byte core matrices), then NX[32], NY[32] of each; a padding row is
+// all zeros and adds exactly 0 to every sum.
 __global__ void k_prep_pack(Pools P) {
     const int a = blockIdx.y;
     if (a >= P.n_active) return;
@@ -302,42 +330,42 @@ __global__ void k_prep_pack(Pools P) {
         cc[k] = 0.5 * (ordered_to_dbl(f.bmin[k]) + ordered_to_dbl(f.bmax[k]));
         if (!isfinite(cc[k])) cc[k] = 0.0;
     }
-    const double c0 = cc[0], c1 = cc[1], c2 = cc[2];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        f.centre[0] = c0;
-        f.centre[1] = c1;
-        f.centre[2] = c2;
+        f.centre[0] = cc[0];
+        f.centre[1] = cc[1];
+        f.centre[2] = cc[2];
     }
     const double fx = f.K[0], fy = f.K[1], cx = f.K[2], cy = f.K[3];
     const double itau = 1.0 / f.tau;
+    const bool tc = f.hr == 1;
     const int64_t npad = (int64_t)f.n_blocks * kSub;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npad;
          i += (int64_t)gridDim.x * blockDim.x) {
-        float v[5];
+        float v[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        const float one = i < f.n ? 1.0f : 0.0f;
         if (i < f.n) {
             const double u = P.uv64[2 * (base + i)], w = P.uv64[2 * (base + i) + 1];
             const double xn = (u - cx) / fx, yn = (w - cy) / fy;
             P.xn64[2 * (base + i)] = xn;
             P.xn64[2 * (base + i) + 1] = yn;
-            v[0] = (float)(P.X64[3 * (base + i)] - c0);
-            v[1] = (float)(P.X64[3 * (base + i) + 1] - c1);
-            v[2] = (float)(P.X64[3 * (base + i) + 2] - c2);
-            v[3] = (float)(-xn * itau);
-            v[4] = (float)(-yn * itau);
-            bool finite = true;
-#pragma unroll
-            for (int k = 0; k < 5; ++k) finite = finite && fabsf(v[k]) <= 0x1p80f;
-            if (!finite) {  // non-finite (never an FP64 inlier) or beyond 2^80: outlier for every pose
-                v[0] = v[1] = v[2] = 0.0f;
-                v[3] = v[4] = 0x1p100f;
-            }
-        } else {
-            v[0] = v[1] = v[2] = v[3] = v[4] = 0.0f;
+            stage_point(P.X64 + 3 * (base + i), xn, yn, cc, itau, v);
         }
         float2 *blk = P.pts32 + (f.blk_off + i / kSub) * kBlockFloat2;
         const int j = (int)(i % kSub);
+        if (tc) {
+            const int t = j >> 5, r = j & 31;
+            char *row = reinterpret_cast<char *>(blk) + t * 1024 + (r >> 3) * 256 + (r & 7) * 16;
+            const float xh = tf32_rn(v[0]), yh = tf32_rn(v[1]), zh = tf32_rn(v[2]);
+            *reinterpret_cast<float4 *>(row) = make_float4(xh, yh, zh, one);
+            *reinterpret_cast<float4 *>(row + 128) =
+                make_float4(tf32_rn(v[0] - xh), tf32_rn(v[1] - yh), tf32_rn(v[2] - zh), 0.0f);
+            float *xy = reinterpret_cast<float *>(blk) + 512 + t * 64 + r;
+            xy[0] = v[3];
+            xy[32] = v[4];
+        } else {
 #pragma unroll
-        for (int k = 0; k < 5; ++k) blk[k * kSub + j] = make_float2(v[k], v[k]);
+            for (int k = 0; k < 5; ++k) blk[k * kSub + j] = make_float2(v[k], v[k]);
+        }
     }
 }
 
@@ -602,13 +630,21 @@ __global__ void k_score_plan(Pools P) {
     int64_t items = 0, parts = 0, hbs = 0;
     int HB = 32, nhb = 0, cb = 1;
     if (act) {
-        HB = 32 * f->hr;
+        HB = f->hr == 1 ? kTcHyp : 32 * f->hr;
         nhb = (f->hyp_count + HB - 1) / HB;
-        // About 8 items per warp slot of the GPU (FP32 kernels, one warp per
-        // item) or per 4 CTA slots (the tensor-core kernel, a CTA per item with
-        // a larger fixed cost per item); at least 2 staging blocks per item.
-        const double target_items = f->hr == 1 ? 8.0 * P.num_sms * 4 : 8.0 * P.num_sms * 16;
-        const double pairs_per_item = fmax((double)pairs_total / target_items, 2.0 * kSub * HB);
+        // FP32 kernels (a warp per item): about 8 items per warp slot, at least
+        // 2 staging blocks each. Tensor-core kernel (a CTA per item, whose fixed
+        // cost is about that of 3 tiles): an item per 16 tiles of a CTA's share,
+        // 1 to 8 a CTA. Measured, 2 / 4 / 8 / 16 items a CTA: 1.2e8 pairs (one
+        // frame) 74 / 78 / 88 / 97 us, 8.0e9 pairs (256 frames, whole run) 3.67 /
+        // 3.68 / 3.60 / 3.67 ms, 8.1e9 (160 frames) 4.10 / 3.68 / 3.58 / 3.65 ms.
+        double slots = 8.0 * P.num_sms * 16, least = 2.0;
+        if (f->hr == 1) {
+            slots = (double)kTcCtas * P.num_sms;
+            slots *= fmin(8.0, fmax(1.0, (double)pairs_total / (slots * HB * kSub * 16)));
+            least = 1.0;
+        }
+        const double pairs_per_item = fmax((double)pairs_total / slots, least * kSub * HB);
         cb = (int)ceil(pairs_per_item / ((double)HB * kSub));
         if (f->chunk_points > 0) cb = max(1, f->chunk_points / kSub);
         cb = max(cb, (f->n_blocks + kMaxScoreChunks - 1) / kMaxScoreChunks);
@@ -871,133 +907,183 @@ __global__ void __launch_bounds__(kScoreWarps * 32) k_score(Pools P) {
 }
 
 // ------------------------------------------------ tensor-core scoring --
-// The same filter with the projection on the 5th-generation tensor cores:
-// for a tile of 128 points and a block of 32 hypotheses, one tcgen05.mma pair
-// (kind::tf32, M = 128 points, N = 96 = z2 | z0 | z1 rows of the 32
-// hypotheses, K = 16 in two steps of 8) writes every z of the tile into tensor
-// memory, and the epilogue (one thread per point) does the reciprocal, the
-// residuals, the saturating r^2 and the sum per hypothesis. TF32 keeps 11 significant bits,
-// so each operand is split into a hi part (rounded to nearest TF32) and the
-// rounded remainder, and the two MMA steps carry all four cross terms: both
-// read the same A row (K = 8), the first with the hi, the second with the lo
+// The same filter with the projection on the 5th-generation tensor cores: for
+// a block of 128 hypotheses and a tile of 32 points, three pairs of
+// tcgen05.mma (kind::tf32, M = 128 hypotheses, N = 32 points, K = 16 in two
+// steps of 8) write every z2, z0 and z1 of the tile into tensor memory, and the
+// epilogue -- one thread per hypothesis -- does the reciprocal, the residuals,
+// the saturating r^2 and its own hypothesis's sum. TF32 keeps 11 significant
+// bits, so each operand is split into a hi part (rounded to nearest TF32) and
+// the rounded remainder, and the two MMA steps carry all four cross terms: both
+// read the same point row (K = 8), the first with the hi, the second with the lo
 // half of the hypothesis row
-//   A row (point)      = [Xh Yh Zh 1 | Xl Yl Zl 0]
-//   B row (hyp. row c) = [ch0..ch3   | ch0..ch2 0 | cl0..cl3   | cl0..cl2 0]
+//   A row (hyp. row c) = [ch0..ch3   | ch0..ch2 0 | cl0..cl3   | cl0..cl2 0]
+//   B row (point)      = [Xh Yh Zh 1 | Xl Yl Zl 0]
 // whose products are exact in FP32 and sum to c . [X 1] with an error of the
 // order of FP32 rounding (the remainders' own rounding is 2^-23 relative).
 // The default scoring shape (FrameDev::hr = 1, points_per_iter = 128).
-constexpr int kTcHyp = 32;        // hypotheses per item (HB at HR = 1)
-constexpr int kTcN = 3 * kTcHyp;   // MMA N: z2 | z0 | z1 rows of the block
-constexpr int kTcPts = 128;       // MMA M: points per tile
-constexpr int kTcThreads = 128;   // one thread per point row of the accumulator
-constexpr int kTcCols = 128;      // tensor-memory columns per CTA (four CTAs per SM at most)
+//
+// Hypotheses are the rows because they stay while the points stream: A is
+// written to tensor memory once per item, each thread its own row; the point
+// tiles are laid out as B operands when a frame is staged (k_prep_pack) and
+// only copied (bulk copies into a ring); and no sum crosses threads but the two
+// point halves of a hypothesis. One warp copies and issues, eight do the
+// epilogue, 8 accumulator columns at a time with the next 8 on their way; the
+// accumulators are released before the last quarter's arithmetic, under which
+// the next tile's MMAs start. What bounds it is the epilogue's instruction
+// issue: per two pairs 2 depth floors, 2 MUFU reciprocals, 2 packed residual FMAs, a
+// packed square, 2 saturating FMAs and a packed add, measured at 9 a pair with
+// register moves, waits and loads. Measured, 8.0e9 pairs of 256 frames: 3.69 ms
+// (2.18e12 pairs/s) against 4.41 ms for points as the rows (a thread per
+// point, 32 hypotheses as columns, A rebuilt and two CTA barriers per tile). Other
+// forms of this one: A in shared memory 3.78 ms; 16 columns at a time 3.78 ms;
+// scalar epilogue 4.13 ms; 16 epilogue warps per CTA 4.44 ms; the last epilogue
+// warp to read a tile issues the next, instead of a warp of its own 4.97 ms;
+// tiles of 32 points, four CTAs per SM 5.74 ms.
+constexpr int kTcPts = kSub;      // MMA N: points per tile, one staging block
+constexpr int kTcWarps = 8;       // epilogue warps: a 32-hypothesis quarter x a 32-point half of the tile each
+constexpr int kTcThreads = 32 * kTcWarps + 32;  // and one warp that copies the points and issues the MMAs
+constexpr int kTcCols = 256;      // tensor-memory columns per CTA (a power of two)
 constexpr int kTcPP = 128;        // points_per_iter value of the shape
-// At most four CTAs per SM (so that 4 x 128 columns never exceed the 512 of an
-// SM and tcgen05.alloc never waits): each asks for more than a fifth of the
-// SM's shared memory. Four CTAs give the epilogue 16 warps per SM.
-constexpr int kTcSmem = 48 * 1024;
-constexpr uint32_t kTcIdesc = (1u << 4)                        // D: F32
-                              | (2u << 7) | (2u << 10)         // A, B: TF32, both K-major
-                              | ((uint32_t)(kTcN >> 3) << 17)  // N
-                              | ((uint32_t)(kTcPts >> 4) << 24);  // M
-// Shared-memory carve-up (bytes): A, B, two point-staging buffers (two
-// blocks each), the cross-warp sums, then barriers and control words.
-constexpr int kTcOffA = 0, kTcOffB = 8192, kTcOffPts = 14336, kTcOffRed = 24576, kTcOffCtl = 25088;
+constexpr int kTcRing = 16;       // staging blocks in flight
+// At most two CTAs per SM (so that 2 x 256 columns never exceed the 512 of an
+// SM and tcgen05.alloc never waits): each asks for more than a third of the
+// SM's shared memory.
+constexpr int kTcSmem = 80 * 1024;
+constexpr uint32_t kTcIdesc = (1u << 4)                          // D: F32
+                              | (2u << 7) | (2u << 10)           // A, B: TF32, both K-major
+                              | ((uint32_t)(kTcPts >> 3) << 17)  // N
+                              | ((uint32_t)(kTcHyp >> 4) << 24);   // M
+// Tensor-memory columns: z2 | z0 | z1 of a tile, then A, 16 (K) a component.
+constexpr int kTcColA = 3 * kTcPts;
+static_assert(kTcColA + 48 <= kTcCols, "tensor-memory carve-up");
+// Shared-memory carve-up (bytes): the point ring, the halves' sums, then
+// barriers and control words.
+constexpr int kTcOffRed = kTcRing * (int)kBlockBytes, kTcOffCtl = kTcOffRed + 4 * kTcHyp;
+static_assert(kTcOffCtl + 256 <= kTcSmem, "shared-memory carve-up");
 
-// Byte offset of element (row r, k) of a K-major operand with 16 K values per
-// row, no swizzle: 8-row x 16-byte core matrices, the four K chunks of a row
-// group adjacent (leading byte offset 128), row groups 512 bytes apart.
-__device__ __forceinline__ int tc_off(int r, int k) {
-    return (((r >> 3) * 4 + (k >> 2)) * 128) + (r & 7) * 16 + (k & 3) * 4;
-}
-// K-major operand with 8 K values per row (two 16-byte K chunks, leading byte
-// offset 128, row groups 256 bytes apart).
-__device__ __forceinline__ int tc_off8(int r, int k) {
-    return (((r >> 3) * 2 + (k >> 2)) * 128) + (r & 7) * 16 + (k & 3) * 4;
-}
+// Shared-memory descriptor of a K-major operand with 8 K values per row, no
+// swizzle: 8-row x 16-byte core matrices, the two K chunks of a row group
+// adjacent (leading byte offset 128), row groups `sbo` bytes apart.
 __device__ __forceinline__ uint64_t tc_desc_sbo(const void *smem, uint32_t sbo) {
     return (uint64_t)((smem_addr(smem) >> 4) & 0x3FFFu) | ((uint64_t)(128 >> 4) << 16) |
            ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
 }
-__device__ __forceinline__ uint64_t tc_desc(const void *smem) {
-    return (uint64_t)((smem_addr(smem) >> 4) & 0x3FFFu) | ((uint64_t)(128 >> 4) << 16) |
-           ((uint64_t)(512 >> 4) << 32) | (1ull << 46);
-}
-__device__ __forceinline__ float tf32_rn(float x) {
-    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
-}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t accumulate) {
     const uint32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(kTcIdesc), "r"(accumulate), "r"(m0), "r"(m1), "r"(m2), "r"(m3));
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b), "r"(kTcIdesc), "r"(accumulate), "r"(m0), "r"(m1), "r"(m2), "r"(m3));
 }
+// 8 columns of this thread's row written.
+__device__ __forceinline__ void tc_st8(uint32_t taddr, const float (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+                 "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
                  : "memory");
 }
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+// 8 accumulator columns of this thread's row.
+__device__ __forceinline__ void tc_ld8(uint32_t taddr, float (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "r"(taddr));
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// B operand of hypothesis block hb: thread t < 32 writes the z2, z0 and z1 rows
-// (t, 32 + t, 64 + t) of hypothesis hb * 32 + t (zero rows past the count).
-__device__ __forceinline__ void tc_build_b(float *sB, const Pools &P, const FrameDev &f, int hb) {
-    const int t = threadIdx.x;
-    if (t >= kTcHyp) return;
-    const int i = hb * kTcHyp + t;
-    const float *src = P.hP32 + 12 * (f.hyp_base + i);
-    float c[12];
-#pragma unroll
-    for (int e = 0; e < 12; ++e) c[e] = i < f.hyp_count ? __ldg(src + e) : 0.0f;
-    char *rb = reinterpret_cast<char *>(sB);
-#pragma unroll
-    for (int comp = 0; comp < 3; ++comp) {
-        const int n = comp * kTcHyp + t;
-        const int cb = comp == 0 ? 8 : (comp == 1 ? 0 : 4);  // z2 | z0 | z1
-        float hi[4], lo[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            hi[k] = tf32_rn(c[cb + k]);
-            lo[k] = tf32_rn(c[cb + k] - hi[k]);
-        }
-        *reinterpret_cast<float4 *>(rb + tc_off(n, 0)) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<float4 *>(rb + tc_off(n, 4)) = make_float4(hi[0], hi[1], hi[2], 0.0f);
-        *reinterpret_cast<float4 *>(rb + tc_off(n, 8)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-        *reinterpret_cast<float4 *>(rb + tc_off(n, 12)) = make_float4(lo[0], lo[1], lo[2], 0.0f);
+// Bounded wait that also gives up once any thread of the CTA has (*err), so an
+// expired wait costs the CTA one time limit, not one per wait.
+__device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, volatile int *err) {
+    if (mbar_wait(bar, parity, 1024)) return true;
+    for (uint32_t k = 1; k < kMaxPolls / 1024; ++k) {
+        if (*err) return false;
+        if (mbar_wait(bar, parity, 1024)) return true;
     }
+    *err = 1;
+    return false;
 }
 
-__global__ void __launch_bounds__(kTcThreads, 4) k_score_tc(Pools P) {
+// A operands of hypothesis block hb into tensor memory (columns from ta, 16 per
+// component): the epilogue warps of half 0 write the hi and those of half 1 the
+// lo halves of the z2, z0 and z1 rows of their lanes' hypotheses (zero rows past
+// the count).
+__device__ __forceinline__ void tc_build_a(uint32_t ta, const Pools &P, const FrameDev &f, int i, bool low) {
+    float c[12];
+    if (i < f.hyp_count) {
+        const float4 *src = reinterpret_cast<const float4 *>(P.hP32 + 12 * (f.hyp_base + i));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float4 v = __ldg(src + k);
+            c[4 * k] = v.x, c[4 * k + 1] = v.y, c[4 * k + 2] = v.z, c[4 * k + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 12; ++e) c[e] = 0.0f;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int comp = 0; comp < 3; ++comp) {
+        const int cb = comp == 0 ? 8 : (comp == 1 ? 0 : 4);  // z2 | z0 | z1
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float hi = tf32_rn(c[cb + k]);
+            v[k] = low ? tf32_rn(c[cb + k] - hi) : hi;
+            v[4 + k] = k < 3 ? v[k] : 0.0f;
+        }
+        tc_st8(ta + 16 * comp + (low ? 8 : 0), v);
+    }
+    tc_wait_st();
+}
+
+// The truncated r^2 of 8 points (accumulator columns z*, offsets at nx / ny)
+// added to a packed sum.
+__device__ __forceinline__ uint64_t tc_points8(const float (&z2)[8], const float (&z0)[8], const float (&z1)[8],
+                                                const ulonglong2 *nx, const ulonglong2 *ny, uint64_t ta) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const ulonglong2 x4 = nx[q], y4 = ny[q];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int p = 4 * q + 2 * h;
+            const uint64_t inv =
+                f2pack(rcp_approx(fmaxf(z2[p], kDepthFloor)), rcp_approx(fmaxf(z2[p + 1], kDepthFloor)));
+            const uint64_t r0 = f2fma(f2pack(z0[p], z0[p + 1]), inv, h ? x4.y : x4.x);
+            const uint64_t r1 = f2fma(f2pack(z1[p], z1[p + 1]), inv, h ? y4.y : y4.x);
+            const uint64_t r1s = f2mul(r1, r1);
+            float r0a, r0b, sa, sb;
+            f2unpack(r0, r0a, r0b);
+            f2unpack(r1s, sa, sb);
+            ta = f2add(ta, f2pack(fma_sat(r0a, r0a, sa), fma_sat(r0b, r0b, sb)));
+        }
+    }
+    return ta;
+}
+
+__global__ void __launch_bounds__(kTcThreads, kTcCtas) k_score_tc(Pools P) {
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    float *sA = reinterpret_cast<float *>(tc_smem + kTcOffA);
-    float *sB = reinterpret_cast<float *>(tc_smem + kTcOffB);
-    float2 *sPts = reinterpret_cast<float2 *>(tc_smem + kTcOffPts);  // 2 buffers x 2 staging blocks
-    float *red = reinterpret_cast<float *>(tc_smem + kTcOffRed);      // [4][32]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(tc_smem + kTcOffCtl);  // points 0, 1; MMA
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(tc_smem + kTcOffCtl + 32);
-    int *ctl = reinterpret_cast<int *>(tc_smem + kTcOffCtl + 48);
-    volatile int *err = reinterpret_cast<volatile int *>(tc_smem + kTcOffCtl + 60);  // a wait gave up
-    long long *run = reinterpret_cast<long long *>(tc_smem + kTcOffCtl + 64);
+    unsigned char *ring = tc_smem;
+    float *red = reinterpret_cast<float *>(tc_smem + kTcOffRed);
+    uint64_t *full = reinterpret_cast<uint64_t *>(tc_smem + kTcOffCtl);  // kTcRing: a block has landed
+    uint64_t *mma = full + kTcRing;        // the tile's accumulators are complete
+    uint64_t *freeb = full + kTcRing + 1;  // every epilogue warp has read them
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(full + kTcRing + 2);
+    int *ctl = reinterpret_cast<int *>(tslot + 1);
+    volatile int *err = ctl + 1;  // a wait gave up
+    long long *run = reinterpret_cast<long long *>(full + kTcRing + 4);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const bool issuer = tid == 32 * kTcWarps;
     if (tid == 0) {
         *err = 0;
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        mbar_init(&bars[2], 1);
+        for (int k = 0; k < kTcRing; ++k) mbar_init(&full[k], 1);
+        mbar_init(mma, 1);
+        mbar_init(freeb, kTcWarps);
         fence_mbar_init();
     }
     if (w == 0) {
@@ -1009,13 +1095,18 @@ __global__ void __launch_bounds__(kTcThreads, 4) k_score_tc(Pools P) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
-    const uint32_t trow = tmem + ((uint32_t)(w * 32) << 16);  // this warp's 32 lanes
-    uint32_t ph0 = 0, ph1 = 0, phm = 0;
+    const int row = (w & 3) * 32 + lane, half = w >> 2;  // epilogue: hypothesis of the block, 32-point half
+    const uint32_t tcol = tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(32 * half);
     const int64_t total = (int64_t)P.counters[kCScoreTotal];
     const int64_t ctas = gridDim.x;
     int cur_a = -1, cur_hb = -1;
     int64_t run_next = 0, run_end = 0;
-    bool ok = true;
+    // The ring's running block count (slot = count % kTcRing, parity =
+    // count / kTcRing) is the tile count: `blk` is the item's first block, the
+    // same in every thread; the issuer's `issued` and `landed` are its copies
+    // started and waited for. The accumulator barriers complete once per tile.
+    uint32_t blk = 0, issued = 0, landed = 0;
+    bool pending = false;  // issuer: an MMA is committed and may be in flight
     for (;;) {
         if (run_next >= run_end) {
             if (tid == 0) {
@@ -1038,156 +1129,139 @@ __global__ void __launch_bounds__(kTcThreads, 4) k_score_tc(Pools P) {
         const int nch = f.n_chunks;
         const int hb = (int)(local / nch), ch = (int)(local % nch);
         const int nh = f.hyp_count;
-        if (a != cur_a || hb != cur_hb) {  // every MMA of the previous item has completed
-            tc_build_b(sB, P, f, hb);
+        const int b0 = ch * f.chunk_blocks;
+        const int nb = min(f.n_blocks - b0, f.chunk_blocks);
+        const unsigned char *g =
+            reinterpret_cast<const unsigned char *>(P.pts32) + (size_t)(f.blk_off + b0) * kBlockBytes;
+        // Every thread is past the previous item: its MMAs have completed and
+        // its ring slots are free.
+        if (issuer) {
+            fence_proxy_async();
+            for (int k = 0; k < min(nb, kTcRing); ++k, ++issued)
+                bulk_load(ring + (issued % kTcRing) * kBlockBytes, g + (size_t)k * kBlockBytes, kBlockBytes,
+                          &full[issued % kTcRing]);
+        }
+        if (a != cur_a || hb != cur_hb) {
+            if (w < kTcWarps)
+                tc_build_a(tmem + ((uint32_t)((w & 3) * 32) << 16) + kTcColA, P, f, hb * kTcHyp + row, half != 0);
             cur_a = a;
             cur_hb = hb;
         }
-        const int b0 = ch * f.chunk_blocks;
-        const int b1 = min(f.n_blocks, b0 + f.chunk_blocks);
-        const int ntiles = (b1 - b0 + 1) / 2;
-        const int64_t fn = f.n;  // read once: the asm barriers below would reload it every tile
-        const float2 *g = P.pts32 + (f.blk_off + b0) * kBlockFloat2;
-        auto tile_blocks = [&](int i) { return min(2, b1 - b0 - 2 * i); };
-        if (tid == 0) {
-            fence_proxy_async();
-            bulk_load(sPts, g, (uint32_t)(tile_blocks(0) * kBlockBytes), &bars[0]);
-            if (ntiles > 1)
-                bulk_load(sPts + 2 * kBlockFloat2, g + 2 * kBlockFloat2, (uint32_t)(tile_blocks(1) * kBlockBytes),
-                          &bars[1]);
-        }
-        uint64_t acc[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) acc[j] = 0ull;
-        // Every thread waits on the copy and MMA barriers itself (two CTA
-        // barriers per tile). A wait that gives up records the error and the
-        // thread carries on through the same barriers, so the CTA leaves the
-        // tile loop together once the error is visible to all.
-        for (int i = 0; i < ntiles; ++i) {
-            const int s = i & 1;
-            if (!*err && !mbar_wait(&bars[s], s ? ph1 : ph0, kMaxPolls)) *err = 1;
-            if (s) ph1 ^= 1u; else ph0 ^= 1u;
-            // A row of this thread's point.
-            const int64_t p0 = (int64_t)(b0 + 2 * i) * kSub;
-            const int cnt = (int)min((int64_t)tile_blocks(i) * kSub, fn - p0);
-            const bool v = tid < cnt;
-            const float2 *tb = sPts + s * 2 * kBlockFloat2 + (tid >> 6) * kBlockFloat2;
-            const int j = tid & (kSub - 1);
-            const float X = v ? tb[j].x : 0.0f, Y = v ? tb[kSub + j].x : 0.0f, Z = v ? tb[2 * kSub + j].x : 0.0f;
-            const float NX = v ? tb[3 * kSub + j].x : 0.0f, NY = v ? tb[4 * kSub + j].x : 0.0f;
-            {
-                const float xh = tf32_rn(X), yh = tf32_rn(Y), zh = tf32_rn(Z);
-                const float xl = tf32_rn(X - xh), yl = tf32_rn(Y - yh), zl = tf32_rn(Z - zh);
-                const float one = v ? 1.0f : 0.0f;
-                // K = 8 (the two MMAs read the same A chunks with the hi and the
-                // lo half of the hypothesis rows): row groups 256 bytes apart.
-                char *ra = reinterpret_cast<char *>(sA);
-                *reinterpret_cast<float4 *>(ra + tc_off8(tid, 0)) = make_float4(xh, yh, zh, one);
-                *reinterpret_cast<float4 *>(ra + tc_off8(tid, 4)) = make_float4(xl, yl, zl, 0.0f);
-            }
-            fence_proxy_async();  // the operands, written by threads, are read by the tensor core
-            __syncthreads();      // the A tile is complete; staging buffer s is free
-            if (tid == 0) {
+        tc_fence_before();
+        __syncthreads();
+        uint64_t sum = 0ull;
+        if (issuer) {
+            // Tile t's six MMAs: z2, z0, z1 into columns 0, 64, 128.
+            const uint64_t dr = tc_desc_sbo(ring, 256);
+            const uint32_t ta = tmem + kTcColA;
+            for (int t = 0; t < nb; ++t) {
+                const uint32_t k = blk + (uint32_t)t;
+                if (tc_wait(&full[k % kTcRing], (k / kTcRing) & 1, err)) ++landed;
+                if (t > 0) {
+                    tc_wait(freeb, (k - 1) & 1, err);
+                    pending = false;
+                }
                 tc_fence_after();
-                const uint64_t da = tc_desc_sbo(sA, 256);
-                tc_mma(tmem, da, tc_desc(sB), 0u);
-                tc_mma(tmem, da, tc_desc(reinterpret_cast<char *>(sB) + 256), 1u);
-                tc_commit(&bars[2]);
-                if (i + 2 < ntiles) {
+                const uint64_t db = dr + (uint64_t)((k % kTcRing) * (kBlockBytes >> 4));
+#pragma unroll
+                for (int comp = 0; comp < 3; ++comp) {
+                    tc_mma(tmem + comp * kTcPts, ta + comp * 16, db, 0u);
+                    tc_mma(tmem + comp * kTcPts, ta + comp * 16 + 8, db, 1u);
+                }
+                tc_commit(mma);
+                pending = true;
+                // The epilogue warps that have read tile t - 1's accumulators are
+                // past tile t - 2's arithmetic: its slot is refilled.
+                if (t >= 2 && t - 2 + kTcRing < nb) {
                     fence_proxy_async();
-                    bulk_load(sPts + s * 2 * kBlockFloat2, g + (int64_t)(2 * (i + 2)) * kBlockFloat2,
-                              (uint32_t)(tile_blocks(i + 2) * kBlockBytes), &bars[s]);
+                    bulk_load(ring + (issued % kTcRing) * kBlockBytes, g + (size_t)(t - 2 + kTcRing) * kBlockBytes,
+                              kBlockBytes, &full[issued % kTcRing]);
+                    ++issued;
                 }
             }
-            if (!*err && !mbar_wait(&bars[2], phm, kMaxPolls)) *err = 1;
-            phm ^= 1u;
-            tc_fence_after();
-            const uint64_t nx2 = f2pack(NX, NX), ny2 = f2pack(NY, NY);
+        } else if (w < kTcWarps) {
+            const bool live = hb * kTcHyp + (w & 3) * 32 < nh;  // a warp past the last hypothesis only keeps step
+            uint64_t acc = 0ull;
+            for (int t = 0; t < nb; ++t) {
+                const uint32_t k = blk + (uint32_t)t;
+                tc_wait(mma, k & 1, err);
+                __syncwarp();
+                tc_fence_after();
+                const unsigned char *xy = ring + (k % kTcRing) * kBlockBytes + 32 * kTcPts + half * 256;
+                const ulonglong2 *nx = reinterpret_cast<const ulonglong2 *>(xy), *ny = nx + 8;
+                float z[2][3][8];
+                uint64_t ta = 0ull;
+                if (live) {
+                    tc_ld8(tcol, z[0][0]);
+                    tc_ld8(tcol + kTcPts, z[0][1]);
+                    tc_ld8(tcol + 2 * kTcPts, z[0][2]);
+                    tc_wait_ld();
 #pragma unroll
-            for (int gq = 0; gq < 2; ++gq) {
-                float z2[16], z0[16], z1[16];
-                tc_ld16(trow + (uint32_t)(16 * gq), z2);
-                tc_ld16(trow + (uint32_t)(kTcHyp + 16 * gq), z0);
-                tc_ld16(trow + (uint32_t)(2 * kTcHyp + 16 * gq), z1);
-                tc_wait_ld();
-                if (v) {
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const float ia = rcp_approx(fmaxf(z2[2 * q], kDepthFloor));
-                        const float ib = rcp_approx(fmaxf(z2[2 * q + 1], kDepthFloor));
-                        const uint64_t inv = f2pack(ia, ib);
-                        const uint64_t r0 = f2fma(f2pack(z0[2 * q], z0[2 * q + 1]), inv, nx2);
-                        const uint64_t r1 = f2fma(f2pack(z1[2 * q], z1[2 * q + 1]), inv, ny2);
-                        const uint64_t r1s = f2mul(r1, r1);
-                        float r0a, r0b, sa, sb;
-                        f2unpack(r0, r0a, r0b);
-                        f2unpack(r1s, sa, sb);
-                        acc[8 * gq + q] = f2add(acc[8 * gq + q], f2pack(fma_sat(r0a, r0a, sa), fma_sat(r0b, r0b, sb)));
+                    for (int q = 0; q < 3; ++q) {
+                        tc_ld8(tcol + 8 * (q + 1), z[(q + 1) & 1][0]);
+                        tc_ld8(tcol + kTcPts + 8 * (q + 1), z[(q + 1) & 1][1]);
+                        tc_ld8(tcol + 2 * kTcPts + 8 * (q + 1), z[(q + 1) & 1][2]);
+                        ta = tc_points8(z[q & 1][0], z[q & 1][1], z[q & 1][2], nx + 2 * q, ny + 2 * q, ta);
+                        tc_wait_ld();
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(freeb);
+                if (live) {
+                    ta = tc_points8(z[1][0], z[1][1], z[1][2], nx + 6, ny + 6, ta);
+                    // Two-level sums: an FP32 lane adds at most 16 values, then
+                    // 32 tile sums, then the item's.
+                    acc = f2add(acc, ta);
+                    if ((t & 31) == 31) {
+                        sum = f2add(sum, acc);
+                        acc = 0ull;
                     }
                 }
             }
-            tc_fence_before();
-            __syncthreads();  // the accumulator and the A tile are free for the next tile
+            sum = f2add(sum, acc);
         }
-        if (*err) ok = false;  // written before the last barrier, so every thread reads the same
-        if (!ok) break;
-        // Chunk partials: the warp's 32 hypotheses over its 32 points (lanes
-        // 2p, 2p + 1 end with hypotheses 2p, 2p + 1), then the four warps in
-        // fixed order.
-#pragma unroll
-        for (int o = 16, m = 8; o >= 2; o >>= 1, m >>= 1) {
-            const bool up = (lane & o) != 0;
-#pragma unroll
-            for (int jj = 0; jj < m; ++jj) {
-                const uint64_t keep = up ? acc[m + jj] : acc[jj];
-                const uint64_t send = up ? acc[jj] : acc[m + jj];
-                acc[jj] = f2add(keep, __shfl_xor_sync(0xffffffffu, send, o));
-            }
-        }
-        acc[0] = f2add(acc[0], __shfl_xor_sync(0xffffffffu, acc[0], 1));
-        if ((lane & 1) == 0) {
-            float lo, hi;
-            f2unpack(acc[0], lo, hi);
-            red[w * kTcHyp + lane] = lo;
-            red[w * kTcHyp + lane + 1] = hi;
-        }
+        blk += (uint32_t)nb;  // (the issuer has started and seen land every block of the item)
+        float lo, hi;
+        f2unpack(sum, lo, hi);
+        float s = lo + hi;
+        if (w < kTcWarps && half) red[row] = s;
         __syncthreads();
-        float *part = P.part + f.part_base;
-        if (tid < kTcHyp) {
-            const int i = hb * kTcHyp + tid;
-            const float s4 = ((red[tid] + red[kTcHyp + tid]) + red[2 * kTcHyp + tid]) + red[3 * kTcHyp + tid];
-            if (i < nh) part[(int64_t)i * nch + ch] = s4;
-        }
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) ctl[2] = (int)atomicAdd(&P.hb_arrive[f.hb_base + hb], 1u);
-        __syncthreads();
-        if (ctl[2] == nch - 1 && tid < kTcHyp) {
+        // Chunk partials; the CTA that completes a block's last chunk sums them
+        // in chunk order.
+        const int i = hb * kTcHyp + row;
+        const bool mine = w < 4 && i < nh;
+        if (mine) s += red[row];
+        bool last = true;
+        if (nch > 1) {
+            float *part = P.part + f.part_base + (int64_t)i * nch;
+            if (mine) part[ch] = s;
             __threadfence();
-            const int i = hb * kTcHyp + tid;
-            if (i < nh) {
-                float s = 0.0f;
-                for (int q = 0; q < nch; ++q) s += __ldcg(part + (int64_t)i * nch + q);
-                P.hS32[f.hyp_base + i] = s;
-                const int64_t sample = P.hId[f.hyp_base + i] >> 2;
-                const int64_t r = (sample - f.step_first) / f.step_div;
-                const unsigned long long key = ((unsigned long long)__float_as_uint(s) << 32) | (unsigned)i;
-                atomicMin(&f.round_min[r], key);
+            __syncthreads();
+            if (tid == 0) ctl[0] = (int)atomicAdd(&P.hb_arrive[f.hb_base + hb], 1u);
+            __syncthreads();
+            last = ctl[0] == nch - 1;
+            if (last && mine) {
+                __threadfence();
+                s = 0.0f;
+                for (int q = 0; q < nch; ++q) s += __ldcg(part + q);
             }
         }
-        __syncthreads();  // red and ctl are reused by the next item
-    }
-    if (!ok) {
-        // Give up: record it and let the copies and the MMA in flight land
-        // (bounded) before the tensor memory is released.
-        if (tid == 0) {
-            flag_error(P, kErrTimeout);
-            // Copies still in flight complete the buffers' current phases; the
-            // last MMA issued completes the phase before the current parity.
-            mbar_wait(&bars[0], ph0, kMaxPolls);
-            mbar_wait(&bars[1], ph1, kMaxPolls);
-            mbar_wait(&bars[2], phm ^ 1u, kMaxPolls);
+        if (last && mine) {
+            P.hS32[f.hyp_base + i] = s;
+            const int64_t sample = P.hId[f.hyp_base + i] >> 2;
+            const int64_t r = (sample - f.step_first) / f.step_div;
+            const unsigned long long key = ((unsigned long long)__float_as_uint(s) << 32) | (unsigned)i;
+            atomicMin(&f.round_min[r], key);
         }
+        if (__syncthreads_or(*err)) break;  // the CTA leaves together
+    }
+    if (issuer && *err) {
+        // Gave up: record it and let the copies and the MMA in flight land
+        // (bounded) before the tensor memory is released.
+        flag_error(P, kErrTimeout);
+        for (; landed != issued; ++landed) mbar_wait(&full[landed % kTcRing], (landed / kTcRing) & 1, kMaxPolls);
+        if (pending) mbar_wait(mma, (blk - 1) & 1, kMaxPolls);
     }
     tc_fence_before();
     __syncthreads();
@@ -2256,10 +2330,10 @@ __global__ void k_debug_counts(Pools P) {
         const double *M = P.hP64 + 12 * (f.hyp_base + h);
         int cnt = 0;
         for (int64_t i = threadIdx.x; i < f.n; i += blockDim.x) {
-            const float2 *blk = P.pts32 + (f.blk_off + i / kSub) * kBlockFloat2;
-            const int j = (int)(i % kSub);
-            const float X = blk[j].x, Y = blk[kSub + j].x, Z = blk[2 * kSub + j].x;
-            const float NX = blk[3 * kSub + j].x, NY = blk[4 * kSub + j].x;
+            float sp[5];
+            stage_point(P.X64 + 3 * (base + i), P.xn64[2 * (base + i)], P.xn64[2 * (base + i) + 1], f.centre,
+                        1.0 / f.tau, sp);
+            const float X = sp[0], Y = sp[1], Z = sp[2], NX = sp[3], NY = sp[4];
             const float z0 = fmaf(Q[0], X, fmaf(Q[1], Y, fmaf(Q[2], Z, Q[3])));
             const float z1 = fmaf(Q[4], X, fmaf(Q[5], Y, fmaf(Q[6], Z, Q[7])));
             const float z2 = fmaf(Q[8], X, fmaf(Q[9], Y, fmaf(Q[10], Z, Q[11])));
