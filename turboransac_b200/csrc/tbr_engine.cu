@@ -168,6 +168,19 @@ static RunOptions make_run_options(const tbr_ransac_options *ro, const tbr_bundl
     return o;
 }
 
+// Whether a call's steps may score in two passes (k_prune): from a round of
+// kPruneMinPairs pairs over the frames that it can help. Each step then decides
+// by its own pairs (kPruneStepPairs); where none does, the two launches cost 6 us a
+// step. One frame, 1000 samples a round, device time without / with: n = 8000 at
+// 10 / 20 / 40 % inliers 532 / 204 / 129 and 463 / 213 / 135 us, n = 12000 694 / 248 /
+// 139 and 543 / 244 / 144, n = 30000 979 / 332 / 199 and 520 / 297 / 203.
+constexpr double kPruneMinPairs = 1.6e7;
+static double prune_pairs(int64_t n, const RunOptions &o) {
+    if (o.hr != 1 || n < kPruneMinPoints) return 0.0;
+    return 1.5 * (double)n * (double)(o.force_samples > 0 ? o.force_samples : o.B);
+}
+static int want_prune(double pairs) { return pairs >= kPruneMinPairs ? 1 : 0; }
+
 class Engine {
    public:
     int device = 0;
@@ -307,7 +320,7 @@ class Engine {
                              3 * (kMaxActive + 1) * 8 + 4096 * 8;
         if (budget < fixed + (64ull << 20)) return fail(TBR_ERR_INVALID_ARG, "workspace too small");
         const size_t rest = budget - fixed;
-        const size_t per_hyp = 96 + 48 + 8 + 4 + 4 * 32 + 4;
+        const size_t per_hyp = 96 + 48 + 8 + 4 + 4 * 32 + 4 + 4;
         P.max_hyps = (int64_t)(rest * 0.3 / per_hyp);
         P.max_hyps = std::max<int64_t>(P.max_hyps, 4096);
         P.max_parts = P.max_hyps * 32;
@@ -345,6 +358,7 @@ class Engine {
         add((void **)&P.hId, 8 * P.max_hyps);
         add((void **)&P.hS32, 4 * P.max_hyps);
         add((void **)&P.part, 4 * P.max_parts);
+        add((void **)&P.surv, 4 * P.max_hyps);
         add((void **)&P.hb_arrive, 4 * P.max_hb);
         add((void **)&P.cHyp, 4 * (size_t)P.cand_cap);
         add((void **)&P.cS64, 8 * (size_t)P.cand_cap);
@@ -477,11 +491,11 @@ class Engine {
     };
     static constexpr const char *kKernelNames[12] = {"k_plan", "k_sample_p3p", "k_score_plan", "k_score",
                                                      "k_select", "k_rescore_plan", "k_rescore", "k_finalize",
-                                                     "k_inliers", "k_lm", "k_prep", "unused"};
+                                                     "k_inliers", "k_lm", "k_prune", "k_score"};
     // Scoring kernel variant: HR hypotheses per lane = 2*HP, PP points per iteration.
-    void launch_score(const Pools &Q, int hr, int pp, cudaStream_t st) {
+    void launch_score(const Pools &Q, int hr, int pp, cudaStream_t st, int pass = 0) {
         const int threads = kScoreWarps * 32;
-        if (hr == 1) k_score_tc<<<kTcCtas * num_sms, kTcThreads, kTcSmem, st>>>(Q);  // (pp == kTcPP)
+        if (hr == 1) k_score_tc<<<kTcCtas * num_sms, kTcThreads, kTcSmem, st>>>(Q, pass);  // (pp == kTcPP)
         else if (hr == 2) k_score<1, 4><<<score_grid[0], threads, 0, st>>>(Q);
         else if (hr == 8) k_score<4, 2><<<score_grid[3], threads, 0, st>>>(Q);
         else if (hr == 6 && pp == 4) k_score<3, 4><<<score_grid[5], threads, 0, st>>>(Q);
@@ -489,20 +503,41 @@ class Engine {
         else if (pp == 4) k_score<2, 4><<<score_grid[2], threads, 0, st>>>(Q);
         else k_score<2, 2><<<score_grid[1], threads, 0, st>>>(Q);
     }
+    // A cluster of 8 CTAs per frame while their number fits the GPU, else of 2 or 1.
+    void launch_prune(const Pools &Q, int n_active, cudaStream_t st) {
+        const unsigned cl = 8 * n_active <= 2 * num_sms ? 8 : (2 * n_active <= 2 * num_sms ? 2 : 1);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(cl * n_active);
+        cfg.blockDim = dim3(1024);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cl;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, k_prune, Q);
+    }
     int pp = kTcPP;  // points per iteration of the scoring kernel (kTcPP: the tensor-core kernel)
 
+    // The planning kernels are one CTA with a thread per frame (and 4 warps at least).
+    static int plan_threads(int n_active) { return std::max(128, (n_active + 31) & ~31); }
     // RANSAC part of a step (plan .. finalize).
     void launch_ransac(const Pools &Q, int n_active, int hr, cudaStream_t st, Profile *prof = nullptr) {
         auto beg = [&](int k) { if (prof) cudaEventRecord(prof->ev[2 * k], st); };
         auto end = [&](int k) { if (prof) { cudaEventRecord(prof->ev[2 * k + 1], st); prof->launches[k]++; } };
-        beg(0); k_plan<<<1, kMaxActive, 0, st>>>(Q); end(0);
+        beg(0); k_plan<<<1, plan_threads(n_active), 0, st>>>(Q); end(0);
         beg(1); k_sample_p3p<<<p3p_grid, 128, 0, st>>>(Q); end(1);
-        beg(2); k_score_plan<<<1, kMaxActive, 0, st>>>(Q); end(2);
+        beg(2); k_score_plan<<<1, plan_threads(n_active), 0, st>>>(Q, 0); end(2);
         beg(3);
         launch_score(Q, hr, pp, st);
         end(3);
+        if (Q.prune) {  // second scoring pass, over what the first leaves
+            beg(10); launch_prune(Q, n_active, st); end(10);
+            beg(11); launch_score(Q, hr, pp, st, 1); end(11);
+        }
         beg(4); k_select<<<n_active, 1024, 0, st>>>(Q); end(4);  // a frame's ~4000 hypotheses: 1024 threads (6.51 ms a batch, 256: 6.59)
-        beg(5); k_rescore_plan<<<1, kMaxActive, 0, st>>>(Q); end(5);
+        beg(5); k_rescore_plan<<<1, plan_threads(n_active), 0, st>>>(Q); end(5);
         beg(6); k_rescore<<<rescore_grid, 256, 0, st>>>(Q); end(6);
         beg(7); k_finalize<<<n_active, 256, 0, st>>>(Q); end(7);
     }
@@ -652,6 +687,7 @@ class Engine {
     // least recently used first.
     struct CachedGraph {
         int n, hr, pp, n_first, bx;  // n_first, bx: split admission (0, 0 without)
+        int prune;
         cudaGraphExec_t exec;
     };
     std::vector<CachedGraph> graph_cache;
@@ -664,7 +700,7 @@ class Engine {
         const int nf = sg ? sg->n_first : 0, bx = sg ? prep_bx(sg->max_n_rest) : 0;
         for (size_t i = 0; i < graph_cache.size(); ++i)
             if (graph_cache[i].n == na && graph_cache[i].hr == hr && graph_cache[i].pp == pp &&
-                graph_cache[i].n_first == nf && graph_cache[i].bx == bx) {
+                graph_cache[i].n_first == nf && graph_cache[i].bx == bx && graph_cache[i].prune == P.prune) {
                 CachedGraph g = graph_cache[i];
                 graph_cache.erase(graph_cache.begin() + i);
                 graph_cache.push_back(g);
@@ -683,7 +719,7 @@ class Engine {
                 cudaGraphExecDestroy(graph_cache.front().exec);
                 graph_cache.erase(graph_cache.begin());
             }
-            graph_cache.push_back({na, hr, pp, nf, bx, exec});
+            graph_cache.push_back({na, hr, pp, nf, bx, P.prune, exec});
         }
         TBR_CUDA(cudaGraphLaunch(exec, stream));
         return TBR_OK;
@@ -702,10 +738,10 @@ class Engine {
             TBR_CUDA(cudaMemcpyAsync(h_counters, Q.counters, 8 * kCNum, cudaMemcpyDeviceToHost, stream));
             TBR_CUDA(cudaStreamSynchronize(stream));
             if (prof)
-                for (int k = 0; k < 10; ++k) {
+                for (int k = 0; k < (Q.prune ? 12 : 10); ++k) {
                     float ms = 0.f;
                     cudaEventElapsedTime(&ms, prof->ev[2 * k], prof->ev[2 * k + 1]);
-                    prof->ms[k] += ms;
+                    prof->ms[k == 11 ? 3 : k] += ms;  // both scoring passes together
                 }
             ++steps;
             if (h_counters[kCError] & kErrTimeout) return fail(TBR_ERR_TIMEOUT, "bounded device wait expired");
@@ -1454,7 +1490,12 @@ static tbr_status enqueue_frames(Engine &E, const std::vector<FrameHost> &fr, co
     TBR_CUDA(cudaSetDevice(E.device));
     TBR_CUDA(cudaMemsetAsync(E.P.counters, 0, 8 * kCNum, E.stream));
     size_t in_bytes = 0;
-    for (auto &f : fr) in_bytes += 40 * (size_t)f.n;
+    double pairs = 0.0;
+    for (auto &f : fr) {
+        in_bytes += 40 * (size_t)f.n;
+        pairs += prune_pairs(f.n, o);
+    }
+    E.P.prune = want_prune(pairs);
     tbr_status st;
     if (!device_points && fr.size() >= 2 && in_bytes >= kStaggerMinBytes) {
         st = admit_host_frames(E, fr, o, slots, max_n, devs, true, !behind);
@@ -1978,6 +2019,12 @@ struct tbr_batch {
     Engine::Profile prof;
 };
 
+static int batch_prune(const tbr_batch *b) {
+    double pairs = 0.0;
+    for (int64_t n : b->ns) pairs += prune_pairs(n, b->o);
+    return want_prune(pairs);
+}
+
 // Live batches. Destroying a context frees the batches made on it; their
 // handles then stay known as dead, so that a later call on one is refused
 // instead of touching freed memory.
@@ -2070,6 +2117,7 @@ tbr_status tbr_batch_create(tbr_context *ctx, const tbr_frame_desc *frames, int3
     b->Q = E.P;
     b->Q.active = b->d_active;
     b->Q.n_active = n_frames;
+    b->Q.prune = batch_prune(b);
     E.launch_prep(b->Q, n_frames, max_n);
     // Snapshot the prepared frame states (AABB centre included).
     for (int i = 0; i < n_frames; ++i)
@@ -2123,11 +2171,17 @@ tbr_status tbr_batch_autotune(tbr_batch *b, int32_t repeats, tbr_tune_entry *ent
     cudaEvent_t t0, t1;
     TBR_CUDA(cudaEventCreate(&t0));
     TBR_CUDA(cudaEventCreate(&t1));
-    auto apply = [&](int hr, int pp, int chunk, cudaGraph_t *g, cudaGraphExec_t *x) -> bool {
+    const RunOptions old = b->o;
+    // Sets the frames' shape; the staging blocks' layout follows its kernel (k_prep_pack).
+    auto set_shape = [&](int hr, int chunk) {
         k_set_shape<<<(n + 127) / 128, 128, 0, E.stream>>>(b->d_init, n, hr, chunk);
-        // The staging blocks' layout follows the shape's kernel (k_prep_pack).
         k_reset_frames<<<n, 128, 0, E.stream>>>(b->Q, b->d_init);
         k_prep_pack<<<dim3(Engine::prep_bx(*std::max_element(b->ns.begin(), b->ns.end())), n), 256, 0, E.stream>>>(b->Q);
+        b->o.hr = hr;
+        b->Q.prune = batch_prune(b);
+    };
+    auto apply = [&](int hr, int pp, int chunk, cudaGraph_t *g, cudaGraphExec_t *x) -> bool {
+        set_shape(hr, chunk);
         if (cudaGetLastError() != cudaSuccess) return false;
         E.pp = pp;
         return E.build_loop_graph(b->Q, n, hr, b->d_init, g, x);
@@ -2165,7 +2219,10 @@ tbr_status tbr_batch_autotune(tbr_batch *b, int32_t repeats, tbr_tune_entry *ent
     }
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
-    if (st) return st;
+    if (st) {  // the batch keeps its graph: its shape again
+        set_shape(old.hr, old.chunk_points);
+        return st;
+    }
     size_t bi = 0;
     for (size_t i = 1; i < tried.size(); ++i)
         if (tried[i].ms < tried[bi].ms) bi = i;
@@ -2173,8 +2230,10 @@ tbr_status tbr_batch_autotune(tbr_batch *b, int32_t repeats, tbr_tune_entry *ent
     // Keep the winner: new initial records and graph for tbr_batch_run.
     cudaGraph_t g = nullptr;
     cudaGraphExec_t x = nullptr;
-    if (!apply(win.hyp_per_thread, win.points_per_iter, win.chunk_points, &g, &x))
+    if (!apply(win.hyp_per_thread, win.points_per_iter, win.chunk_points, &g, &x)) {
+        set_shape(old.hr, old.chunk_points);
         return fail(TBR_ERR_CUDA, "autotune graph capture failed");
+    }
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     b->graph = g;
@@ -2251,7 +2310,7 @@ tbr_status tbr_batch_profile(tbr_batch *b, tbr_kernel_profile *out, int32_t max,
     if (st) return st;
     if (pairs_scored) *pairs_scored = E.h_counters[kCPairsTotal];
     int m = 0;
-    for (int k = 0; k < 10 && m < max; ++k, ++m) {
+    for (int k = 0; k < (b->Q.prune ? 11 : 10) && m < max; ++k, ++m) {
         std::snprintf(out[m].name, sizeof(out[m].name), "%s", Engine::kKernelNames[k]);
         out[m].total_ms = pr.ms[k];
         out[m].launches = pr.launches[k];
@@ -2569,6 +2628,9 @@ static tbr_status server_step(tbr_server *s) {
         }
         TBR_CUDA(cudaMemcpyAsync(E.d_active, ha, 4 * na, cudaMemcpyHostToDevice, E.stream));
         E.P.n_active = na;
+        double pairs = 0.0;
+        for (auto &r : s->resident) pairs += prune_pairs(r.req->n, s->o);
+        E.P.prune = want_prune(pairs);
         if (na >= kServerOverlapFrames) {
             // Many resident frames: the refinement of frames that finished RANSAC
             // in earlier steps runs beside this step's RANSAC (disjoint frames);
@@ -2850,9 +2912,10 @@ tbr_status tbr_debug_score_samples(tbr_context *ctx, const double *points2D, con
     tbr_status st = admit_frames(E, {fh}, o, slots, max_n);
     if (st) return st;
     E.launch_prep(1, max_n);
+    E.P.prune = 0;  // every hypothesis's score is wanted
     k_plan<<<1, kMaxActive, 0, E.stream>>>(E.P);
     k_sample_p3p<<<E.p3p_grid, 128, 0, E.stream>>>(E.P);
-    k_score_plan<<<1, kMaxActive, 0, E.stream>>>(E.P);
+    k_score_plan<<<1, kMaxActive, 0, E.stream>>>(E.P, 0);
     E.launch_score(E.P, o.hr, o.pp, E.stream);
     if (counts) k_debug_counts<<<E.num_sms * 4, 256, 0, E.stream>>>(E.P);
     TBR_CUDA(cudaGetLastError());

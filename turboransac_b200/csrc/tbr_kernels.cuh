@@ -5,7 +5,9 @@
 //   k_plan          rounds to run this step per frame (adaptive-termination aware)
 //   k_sample_p3p    one thread per minimal sample: Philox triple (or replay), FP64 P3P
 //   k_score_plan    work items (frame, 32*HR hypotheses, point chunk)
-//   k_score         FP32 truncated-MSAC filter pass (the hot kernel)
+//   k_score_tc / k_score   FP32 truncated-MSAC filter pass (the hot kernel)
+//   k_prune         drops hypotheses that a random sample of the points rules out;
+//                   the rest are scored on the other points (a second pass)
 //   k_select        candidates within a safe band of each round's running minimum
 //   k_rescore_plan / k_rescore   exact FP64 MSAC of the candidates (reference formula)
 //   k_finalize      the reference's selection and stop rule, round by round
@@ -35,6 +37,13 @@ constexpr int kMaxRChunks = 32;                   // FP64 rescoring point chunks
 constexpr int kMaxScoreChunks = 64;               // FP32 scoring point chunks per frame
 constexpr int kMaxActive = 1024;                  // frames advanced by one step
 constexpr uint32_t kMaxPolls = 1u << 26;          // bounded mbarrier waits (~seconds)
+// Scoring in two passes (k_prune): frames from kPruneMinPoints points stage them in
+// a random order; the first pass scores every hypothesis on a prefix of it.
+constexpr int kPruneMinPoints = 1024;
+// A step is scored in two passes from this many pairs on: it costs two launches
+// (about 10 us for one frame), the time of about this many pairs.
+constexpr unsigned long long kPruneStepPairs = 45000000ull;
+constexpr float kPruneLog = 46.0f;                // -ln of a hypothesis's chance to be dropped wrongly (< 2^-64)
 constexpr int kScoreWarps = 4;                    // warps per scoring CTA
 constexpr int kTcCtas = 2;                          // ... and its CTAs per SM (tensor memory)
 constexpr int kTcHyp = 128;                       // tensor-core scoring: hypotheses per item (MMA M), a thread each
@@ -68,6 +77,8 @@ enum Counter : int {
     kCLMPending,
     kCWorkPairs,
     kCCandNext,
+    kCTwoPass,  // pairs of the step's frames that are scored in two passes (0: none is)
+    kCPruned,   // CTAs of k_prune that are done
     kCSteps,
     kCPairsTotal,
     kCNum
@@ -133,10 +144,11 @@ struct __align__(16) FrameDev {
     int32_t hyp_count, n_hblocks;
     int32_t n_chunks, chunk_blocks;
     int64_t part_base, hb_base;
+    int32_t m_blocks, surv;  // two-pass scoring: staging blocks of the first pass (0: one pass over all);
+                             // hypotheses left for the second (Pools::surv)
     int32_t cand_count, n_rchunks;
     int64_t rchunk, cand_base;
     unsigned long long round_min[kMaxRoundsPerStep];
-    int32_t round_hyps[kMaxRoundsPerStep];
     // ---- LM ----
     int64_t num_inliers;
     int64_t lm_epoch;  // engine step in which RANSAC finished
@@ -170,6 +182,9 @@ struct Pools {
     int64_t *hId;
     float *hS32;
     float *part;
+    int32_t *surv;       // two-pass scoring: a frame's hypotheses left, from its hyp_base
+    int32_t prune;       // 1: the step has a second scoring pass
+    int32_t pad0;
     unsigned *hb_arrive;
     int64_t max_hyps, max_parts, max_hb;
     // FP64 re-rank candidates: one pool shared by the step, a region per frame
@@ -263,6 +278,37 @@ __device__ __forceinline__ void flag_error(const Pools &P, unsigned long long bi
     atomicOr(&P.counters[kCError], bits);
 }
 
+// Position of point i in a frame's staging order: a bijection on [0, n) keyed by
+// the frame's seed (six rounds of odd multiply, add and xor-shift on the next
+// power of two, walked along its cycle until it falls below n).
+__device__ __forceinline__ uint32_t stage_position(uint32_t i, uint32_t n, uint64_t seed) {
+    const int bits = 32 - __clz(n - 1);
+    const uint32_t mask = bits >= 32 ? 0xFFFFFFFFu : (1u << bits) - 1u;
+    const int sh = (bits + 1) / 2;
+    uint32_t x = i;
+    do {
+        uint64_t z = seed;
+#pragma unroll
+        for (int r = 0; r < 6; ++r) {
+            // SplitMix64 (Steele, Lea, Flood, OOPSLA 2014): the round's odd factor and addend.
+            z += 0x9E3779B97F4A7C15ull;
+            uint64_t k = z;
+            k = (k ^ (k >> 30)) * 0xBF58476D1CE4E5B9ull;
+            k = (k ^ (k >> 27)) * 0x94D049BB133111EBull;
+            k ^= k >> 31;
+            x = (x * ((uint32_t)k | 1u) + (uint32_t)(k >> 32)) & mask;
+            x ^= x >> sh;
+        }
+    } while (x >= n);
+    return x;
+}
+
+// Round, within the step, of the hypothesis with the given id (a step draws
+// fewer than 2^32 samples).
+__device__ __forceinline__ int round_of(const FrameDev &f, int64_t id) {
+    return f.step_rounds <= 1 ? 0 : (int)((uint32_t)((id >> 2) - f.step_first) / (uint32_t)f.step_div);
+}
+
 // ----------------------------------------------------------- admission -----
 // AABB of the frame's world points (ordered-integer atomics: order independent).
 __global__ void k_prep_bounds(Pools P) {
@@ -319,7 +365,8 @@ __device__ __forceinline__ void stage_point(const double *X, double xn, double y
 // that one 64-bit lane pair feeds both halves of a packed FP32x2 instruction.
 // Tensor-core kernel: two 32-point B operands ([hi xyz, 1 | lo xyz, 0] rows in
 // 8-row x 16-byte core matrices), then NX[32], NY[32] of each; a padding row is
-// all zeros and adds exactly 0 to every sum.
+// all zeros and adds exactly 0 to every sum. Frames large enough for two-pass
+// scoring (k_prune) are staged in a random order.
 __global__ void k_prep_pack(Pools P) {
     const int a = blockIdx.y;
     if (a >= P.n_active) return;
@@ -338,6 +385,7 @@ __global__ void k_prep_pack(Pools P) {
     const double fx = f.K[0], fy = f.K[1], cx = f.K[2], cy = f.K[3];
     const double itau = 1.0 / f.tau;
     const bool tc = f.hr == 1;
+    const bool mixed = tc && f.n >= kPruneMinPoints && f.n < (1ll << 31);
     const int64_t npad = (int64_t)f.n_blocks * kSub;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npad;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -350,8 +398,9 @@ __global__ void k_prep_pack(Pools P) {
             P.xn64[2 * (base + i) + 1] = yn;
             stage_point(P.X64 + 3 * (base + i), xn, yn, cc, itau, v);
         }
-        float2 *blk = P.pts32 + (f.blk_off + i / kSub) * kBlockFloat2;
-        const int j = (int)(i % kSub);
+        const int64_t at = mixed && i < f.n ? stage_position((uint32_t)i, (uint32_t)f.n, f.seed) : i;
+        float2 *blk = P.pts32 + (f.blk_off + at / kSub) * kBlockFloat2;
+        const int j = (int)(at % kSub);
         if (tc) {
             const int t = j >> 5, r = j & 31;
             char *row = reinterpret_cast<char *>(blk) + t * 1024 + (r >> 3) * 256 + (r & 7) * 16;
@@ -478,6 +527,8 @@ __global__ void k_plan(Pools P) {
         P.counters[kCScoreNext] = 0;
         P.counters[kCRescoreNext] = 0;
         P.counters[kCCandNext] = 0;
+        P.counters[kCTwoPass] = 0;
+        P.counters[kCPruned] = 0;
         P.counters[kCStillRansac] = 0;
         P.counters[kCLMPending] = 0;
     }
@@ -613,17 +664,65 @@ __global__ void __launch_bounds__(128) k_sample_p3p(Pools P) {
 }
 
 // ------------------------------------------------------------ scoring -----
+// Staging blocks of a frame's first scoring pass; 0: one pass over all of them.
+// With a best model from earlier steps the prefix is long enough that a
+// hypothesis without inliers is ruled out by it with a third to spare (see
+// k_prune: a prefix of m points can rule out a gain of mu from
+// m >= kPruneLog / mu on). Without one it is a quarter of the points, 512 to 1024.
+// A prefix of more than half the points is not worth a second pass.
+__device__ __forceinline__ int first_pass_blocks(const FrameDev &f) {
+    if (f.hr != 1 || f.n < kPruneMinPoints || f.n >= (1ll << 31)) return 0;
+    const float n = (float)f.n;
+    float m = fminf(fmaxf(0.25f * n, 512.0f), 1024.0f);
+    if (f.found) {
+        const float mu = 1.0f - (float)(f.best_score / f.sq_thr) * (1.0f + 1.0f / 2048.0f) / n - 2.0f / n;
+        if (!(mu > 0.0f)) return 0;
+        m = fmaxf(512.0f, (4.0f / 3.0f) * kPruneLog / mu);
+    }
+    if (!(2.0f * m <= n)) return 0;
+    return ((int)m + kSub - 1) / kSub;
+}
+
 // Work items: (frame, block of 32*HR hypotheses, point chunk). Chunks are sized
-// so that the step has enough items to keep every SM busy.
-__global__ void k_score_plan(Pools P) {
+// so that the step has enough items to keep every SM busy. Pass 0 covers every
+// hypothesis and the points of its first pass, pass 1 the hypotheses left by
+// k_prune and the other points.
+__device__ __forceinline__ void score_plan(const Pools &P, int pass) {
     __shared__ int64_t sh[33];
     __shared__ unsigned long long pairs_total;
     const int a = threadIdx.x;
     FrameDev *f = a < P.n_active ? &P.frames[P.active[a]] : nullptr;
-    const bool act = f && f->step_samples > 0;
+    bool act = f && f->step_samples > 0;
     if (a == 0) pairs_total = 0;
+    int hyps = 0, blocks = 0;  // of this pass
+    __shared__ unsigned long long two_pass;  // pairs of the frames that could be scored in two passes
+    if (pass == 0 && P.prune) {
+        if (a == 0) two_pass = 0;
+        __syncthreads();
+        if (act) {
+            f->m_blocks = first_pass_blocks(*f);
+            if (f->m_blocks)
+                atomicAdd(&two_pass, (unsigned long long)f->hyp_count * (unsigned long long)f->n);
+        }
+        __syncthreads();
+    }
+    if (act) {
+        if (pass == 0) {
+            hyps = f->hyp_count;
+            if (!P.prune || two_pass < kPruneStepPairs) f->m_blocks = 0;
+            f->surv = 0;
+            blocks = f->m_blocks ? f->m_blocks : f->n_blocks;
+        } else {
+            act = f->m_blocks > 0;
+            hyps = f->surv;
+            blocks = f->n_blocks - f->m_blocks;
+        }
+    }
     __syncthreads();
-    if (act) atomicAdd(&pairs_total, (unsigned long long)f->hyp_count * (unsigned long long)f->n);
+    if (act) {
+        const int64_t n = pass ? f->n - (int64_t)f->m_blocks * kSub : min(f->n, (int64_t)blocks * kSub);
+        atomicAdd(&pairs_total, (unsigned long long)hyps * (unsigned long long)n);
+    }
     __syncthreads();
     __shared__ unsigned long long parts_total;
     if (a == 0) parts_total = 0;
@@ -631,7 +730,7 @@ __global__ void k_score_plan(Pools P) {
     int HB = 32, nhb = 0, cb = 1;
     if (act) {
         HB = f->hr == 1 ? kTcHyp : 32 * f->hr;
-        nhb = (f->hyp_count + HB - 1) / HB;
+        nhb = (hyps + HB - 1) / HB;
         // FP32 kernels (a warp per item): about 8 items per warp slot, at least
         // 2 staging blocks each. Tensor-core kernel (a CTA per item, whose fixed
         // cost is about that of 3 tiles): an item per 16 tiles of a CTA's share,
@@ -647,9 +746,9 @@ __global__ void k_score_plan(Pools P) {
         const double pairs_per_item = fmax((double)pairs_total / slots, least * kSub * HB);
         cb = (int)ceil(pairs_per_item / ((double)HB * kSub));
         if (f->chunk_points > 0) cb = max(1, f->chunk_points / kSub);
-        cb = max(cb, (f->n_blocks + kMaxScoreChunks - 1) / kMaxScoreChunks);
-        cb = max(1, min(cb, f->n_blocks));
-        atomicAdd(&parts_total, (unsigned long long)f->hyp_count * ((f->n_blocks + cb - 1) / cb));
+        cb = max(cb, (blocks + kMaxScoreChunks - 1) / kMaxScoreChunks);
+        cb = max(1, min(cb, blocks));
+        atomicAdd(&parts_total, (unsigned long long)hyps * ((blocks + cb - 1) / cb));
     }
     __syncthreads();
     if (act) {
@@ -657,27 +756,30 @@ __global__ void k_score_plan(Pools P) {
         const unsigned long long pt = parts_total;
         if (pt > (unsigned long long)P.max_parts) {
             const int scale = (int)((pt + P.max_parts - 1) / P.max_parts);
-            cb = min(f->n_blocks, cb * scale);
+            cb = min(blocks, cb * scale);
         }
-        const int nch = (f->n_blocks + cb - 1) / cb;
+        const int nch = (blocks + cb - 1) / cb;
         f->n_hblocks = nhb;
         f->chunk_blocks = cb;
         f->n_chunks = nch;
         items = (int64_t)nhb * nch;
-        parts = (int64_t)f->hyp_count * nch;
+        parts = (int64_t)hyps * nch;
         hbs = nhb;
     }
-    // Round minima of every planned frame, reset by the whole block.
-    for (int idx = threadIdx.x; idx < P.n_active * kMaxRoundsPerStep; idx += blockDim.x) {
-        FrameDev &g = P.frames[P.active[idx / kMaxRoundsPerStep]];
-        if (g.step_samples > 0) g.round_min[idx % kMaxRoundsPerStep] = ~0ull;
+    // Round minima of every planned frame's rounds, reset a warp per frame.
+    for (int k = threadIdx.x >> 5; k < P.n_active; k += blockDim.x >> 5) {
+        FrameDev &g = P.frames[P.active[k]];
+        if (g.step_samples > 0 && (pass == 0 || g.m_blocks > 0))
+            for (int r = threadIdx.x & 31; r < (int)g.step_rounds; r += 32) g.round_min[r] = ~0ull;
     }
     int64_t tot;
     const int64_t iexcl = block_exclusive_scan(items, sh, tot);
     if (a < P.n_active) P.item_prefix[a] = iexcl;
     if (a == 0) {
+        if (pass == 0 && P.prune && two_pass >= kPruneStepPairs) P.counters[kCTwoPass] = two_pass;
         P.item_prefix[P.n_active] = tot;
         P.counters[kCScoreTotal] = (unsigned long long)tot;
+        P.counters[kCScoreNext] = 0;
         P.counters[kCWorkPairs] = pairs_total;
         P.counters[kCPairsTotal] += pairs_total;
     }
@@ -690,6 +792,7 @@ __global__ void k_score_plan(Pools P) {
     for (int64_t i = threadIdx.x; i < min(tot, P.max_hb); i += blockDim.x) P.hb_arrive[i] = 0;
     if (a == 0 && tot > P.max_hb) flag_error(P, kErrOverflow);
 }
+__global__ void k_score_plan(Pools P, int pass) { score_plan(P, pass); }
 
 // Per (hypothesis, point) the FP32 filter accumulates min(r^2 / tau^2, 1),
 // counting a point with non-positive depth as an outlier (msac.cuh:46
@@ -896,11 +999,9 @@ __global__ void __launch_bounds__(kScoreWarps * 32) k_score(Pools P) {
                 float s = 0.0f;
                 for (int q = 0; q < nch; ++q) s += __ldcg(part + (int64_t)i * nch + q);
                 P.hS32[hbase + i] = s;
-                const int64_t sample = P.hId[hbase + i] >> 2;
-                const int64_t r = (sample - f.step_first) / f.step_div;
                 const unsigned long long key =
                     ((unsigned long long)__float_as_uint(s) << 32) | (unsigned)i;
-                atomicMin(&f.round_min[r], key);
+                atomicMin(&f.round_min[round_of(f, P.hId[hbase + i])], key);
             }
         }
     }
@@ -1009,13 +1110,13 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, volatile
     return false;
 }
 
-// A operands of hypothesis block hb into tensor memory (columns from ta, 16 per
+// A operands of a hypothesis block into tensor memory (columns from ta, 16 per
 // component): the epilogue warps of half 0 write the hi and those of half 1 the
-// lo halves of the z2, z0 and z1 rows of their lanes' hypotheses (zero rows past
-// the count).
+// lo halves of the z2, z0 and z1 rows of their lanes' hypotheses i (zero rows
+// where i < 0).
 __device__ __forceinline__ void tc_build_a(uint32_t ta, const Pools &P, const FrameDev &f, int i, bool low) {
     float c[12];
-    if (i < f.hyp_count) {
+    if (i >= 0) {
         const float4 *src = reinterpret_cast<const float4 *>(P.hP32 + 12 * (f.hyp_base + i));
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -1066,7 +1167,8 @@ __device__ __forceinline__ uint64_t tc_points8(const float (&z2)[8], const float
     return ta;
 }
 
-__global__ void __launch_bounds__(kTcThreads, kTcCtas) k_score_tc(Pools P) {
+__global__ void __launch_bounds__(kTcThreads, kTcCtas) k_score_tc(Pools P, int pass) {
+    if (pass && P.counters[kCTwoPass] == 0) return;
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     unsigned char *ring = tc_smem;
     float *red = reinterpret_cast<float *>(tc_smem + kTcOffRed);
@@ -1128,9 +1230,12 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) k_score_tc(Pools P) {
         const int64_t local = item - P.item_prefix[a];
         const int nch = f.n_chunks;
         const int hb = (int)(local / nch), ch = (int)(local % nch);
-        const int nh = f.hyp_count;
-        const int b0 = ch * f.chunk_blocks;
-        const int nb = min(f.n_blocks - b0, f.chunk_blocks);
+        // Pass 0: every hypothesis, the first pass's blocks; pass 1: the ones left, the others.
+        const int nh = pass ? f.surv : f.hyp_count;
+        const int b0 = (pass ? f.m_blocks : 0) + ch * f.chunk_blocks;
+        const int nb = min((pass || !f.m_blocks ? f.n_blocks : f.m_blocks) - b0, f.chunk_blocks);
+        const int i = hb * kTcHyp + row;  // this thread's hypothesis: its place in the pass, its index
+        const int hi = i >= nh ? -1 : (pass ? P.surv[f.hyp_base + i] : i);
         const unsigned char *g =
             reinterpret_cast<const unsigned char *>(P.pts32) + (size_t)(f.blk_off + b0) * kBlockBytes;
         // Every thread is past the previous item: its MMAs have completed and
@@ -1143,7 +1248,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) k_score_tc(Pools P) {
         }
         if (a != cur_a || hb != cur_hb) {
             if (w < kTcWarps)
-                tc_build_a(tmem + ((uint32_t)((w & 3) * 32) << 16) + kTcColA, P, f, hb * kTcHyp + row, half != 0);
+                tc_build_a(tmem + ((uint32_t)((w & 3) * 32) << 16) + kTcColA, P, f, hi, half != 0);
             cur_a = a;
             cur_hb = hb;
         }
@@ -1222,15 +1327,14 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) k_score_tc(Pools P) {
             sum = f2add(sum, acc);
         }
         blk += (uint32_t)nb;  // (the issuer has started and seen land every block of the item)
-        float lo, hi;
-        f2unpack(sum, lo, hi);
-        float s = lo + hi;
+        float s, s1;
+        f2unpack(sum, s, s1);
+        s += s1;
         if (w < kTcWarps && half) red[row] = s;
         __syncthreads();
         // Chunk partials; the CTA that completes a block's last chunk sums them
-        // in chunk order.
-        const int i = hb * kTcHyp + row;
-        const bool mine = w < 4 && i < nh;
+        // in chunk order, after the first pass's sum in the second.
+        const bool mine = w < 4 && hi >= 0;
         if (mine) s += red[row];
         bool last = true;
         if (nch > 1) {
@@ -1248,11 +1352,10 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) k_score_tc(Pools P) {
             }
         }
         if (last && mine) {
-            P.hS32[f.hyp_base + i] = s;
-            const int64_t sample = P.hId[f.hyp_base + i] >> 2;
-            const int64_t r = (sample - f.step_first) / f.step_div;
-            const unsigned long long key = ((unsigned long long)__float_as_uint(s) << 32) | (unsigned)i;
-            atomicMin(&f.round_min[r], key);
+            if (pass) s += P.hS32[f.hyp_base + hi];
+            P.hS32[f.hyp_base + hi] = s;
+            const unsigned long long key = ((unsigned long long)__float_as_uint(s) << 32) | (unsigned)hi;
+            atomicMin(&f.round_min[round_of(f, P.hId[f.hyp_base + hi])], key);
         }
         if (__syncthreads_or(*err)) break;  // the CTA leaves together
     }
@@ -1266,6 +1369,158 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) k_score_tc(Pools P) {
     tc_fence_before();
     __syncthreads();
     if (w == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTcCols));
+}
+
+// --------------------------------------------------------------- pruning --
+// Between the two scoring passes of a frame: which hypotheses can still win.
+//
+// A point's gain is 1 - min(r^2 / tau^2, 1), in [0, 1]; a hypothesis with mean
+// gain mu over the n points has the score n (1 - mu). The staging order is a random
+// permutation (stage_position) that depends on neither the points' values nor the
+// hypotheses, so the first pass's points are a uniform sample without
+// replacement, and by Hoeffding (1963, theorems 1 and 4) a hypothesis with
+// mean gain >= mu has a sample mean <= x < mu with probability at most
+// exp(-m KL(x || mu)), KL the Bernoulli relative entropy. Let T bound the
+// running best score of a round from above: the best of earlier steps, and the
+// full scores -- computed here -- of this and earlier rounds' leaders after
+// the first pass. A hypothesis matters only if its score is inside the candidate
+// band of the running best (k_select), i.e. its mean gain is at least
+// mu = 1 - (T + T/2048 + 2) / n, the band taken wide enough for both FP32 sums. It
+// is dropped when its sample mean has KL(x || mu) >= kPruneLog / m: a hypothesis
+// that matters is dropped with probability < exp(-46) < 2^-64. The others,
+// typically a few percent, are scored on the remaining points.
+//
+// A cluster of CTAs per frame (one CTA each with many frames): the leader's points
+// and the hypotheses are shared out over it; the launch's last CTA to finish plans
+// the second pass. What bounds it is latency. Measured, one pass -> two: 256 frames
+// 8.0e9 -> 1.3e9 pairs, scoring 3.60 -> 1.07 ms, this kernel 5 x 40 us, whole run 5.35 ->
+// 3.07 ms; one frame of 50000 points at 8 % inliers 4.0e9 -> 4.7e8 pairs, 3.33 -> 2.00
+// ms; the candidates re-ranked are the same ones.
+__device__ __forceinline__ float bernoulli_kl(float x, float mu) {
+    const float a = x > 0.0f ? x * logf(x / mu) : 0.0f;
+    return a + (1.0f - x) * (log1pf(-x) - log1pf(-mu));
+}
+
+__global__ void __launch_bounds__(1024) k_prune(Pools P) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ float cut[kMaxRoundsPerStep];
+    __shared__ float wsum[32], csum;
+    __shared__ int fill, base, last;
+    if (P.counters[kCTwoPass] == 0) return;
+    const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    FrameDev &f = P.frames[P.active[blockIdx.x / CL]];
+    const bool act = f.status == kRansac && f.step_samples > 0 && f.m_blocks > 0;  // uniform over the cluster
+    if (act) {
+        const int R = (int)f.step_rounds;
+        const float n = (float)f.n, m = (float)(f.m_blocks * kSub);
+        const float inf = __int_as_float(0x7f800000);
+        // The bound: the best of earlier steps, or -- without one -- the full
+        // score of the first round's leader from that round on.
+        const bool found = f.found != 0;
+        float T = found ? (float)(f.best_score / f.sq_thr) : inf;
+        int from = 0;                 // first round that T bounds
+        unsigned leader = 0xFFFFFFFFu;
+        if (!found) {
+            unsigned long long key = ~0ull;
+            for (; from < R && (key = f.round_min[from]) == ~0ull; ++from) {}
+            if (from < R) {
+                leader = (unsigned)key;
+                const float *Q = P.hP32 + 12 * (f.hyp_base + (int64_t)leader);
+                float c[12];
+#pragma unroll
+                for (int e = 0; e < 12; ++e) c[e] = __ldg(Q + e);
+                float sum = 0.0f;
+#pragma unroll 2
+                for (int p = f.m_blocks * kSub + rank * (int)blockDim.x + tid; p < (int)f.n; p += CL * blockDim.x) {
+                    const char *blk = reinterpret_cast<const char *>(P.pts32 + (f.blk_off + p / kSub) * kBlockFloat2);
+                    const int j = p % kSub;
+                    const char *row = blk + (j >> 3) * 256 + (j & 7) * 16;
+                    const float4 h = *reinterpret_cast<const float4 *>(row);
+                    const float4 l = *reinterpret_cast<const float4 *>(row + 128);
+                    const float *xy = reinterpret_cast<const float *>(blk) + 512 + (j >> 5) * 64 + (j & 31);
+                    const float X = h.x + l.x, Y = h.y + l.y, Z = h.z + l.z;
+                    const float z0 = fmaf(c[0], X, fmaf(c[1], Y, fmaf(c[2], Z, c[3])));
+                    const float z1 = fmaf(c[4], X, fmaf(c[5], Y, fmaf(c[6], Z, c[7])));
+                    const float z2 = fmaf(c[8], X, fmaf(c[9], Y, fmaf(c[10], Z, c[11])));
+                    const float inv = rcp_approx(fmaxf(z2, kDepthFloor));
+                    const float r0 = fmaf(z0, inv, xy[0]), r1 = fmaf(z1, inv, xy[32]);
+                    sum += fma_sat(r0, r0, r1 * r1);
+                }
+                sum = warp_sum(sum);
+                if (lane == 0) wsum[w] = sum;
+                __syncthreads();
+                if (tid == 0) {
+                    float s = 0.0f;
+                    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += wsum[q];
+                    csum = s;
+                }
+                cluster.sync();
+                T = __uint_as_float((unsigned)(key >> 32));
+                for (int q = 0; q < CL; ++q) T += *cluster.map_shared_rank(&csum, q);
+            }
+        }
+        // The sample sum from which a hypothesis is dropped: the largest x with
+        // m KL(x || mu) >= kPruneLog by bisection (12 steps, the safe end), with a
+        // margin for the FP32 sum.
+        if (w == 0) {
+            const float mu = 1.0f - T * (1.0f + 1.0f / 2048.0f) / n - 2.0f / n;
+            float c = inf;
+            if (mu > 0.0f && m * bernoulli_kl(0.0f, mu) >= kPruneLog) {
+                float lo = 0.0f, hi = mu;
+                for (int it = 0; it < 12; ++it) {
+                    const float x = 0.5f * (lo + hi);
+                    if (m * bernoulli_kl(x, mu) >= kPruneLog) lo = x; else hi = x;
+                }
+                c = m * (1.0f - lo) + m * 2e-5f;
+            }
+            for (int r = lane; r < R; r += 32) cut[r] = r >= from ? c : inf;
+        }
+        __syncthreads();
+        // Each CTA keeps from its slice of the hypotheses, four a thread at a time.
+        const int nh = f.hyp_count;
+        const int64_t hb = f.hyp_base;
+        const int i1 = (int)((int64_t)nh * (rank + 1) / CL);
+        for (int i0 = (int)((int64_t)nh * rank / CL); i0 < i1; i0 += 4 * blockDim.x) {
+            unsigned keep = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * (int)blockDim.x + tid;
+                if (i < i1 && (P.hS32[hb + i] < cut[R == 1 ? 0 : round_of(f, P.hId[hb + i])] || (unsigned)i == leader))
+                    keep |= 1u << u;
+            }
+            if (tid == 0) fill = 0;
+            __syncthreads();
+            const int mine = __popc(keep);
+            int at = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, at, o);
+                if (lane >= o) at += u;
+            }
+            int w0 = 0;
+            if (lane == 31 && at) w0 = atomicAdd(&fill, at);
+            w0 = __shfl_sync(0xffffffffu, w0, 31);
+            __syncthreads();
+            if (tid == 0) base = fill ? atomicAdd(&f.surv, fill) : 0;
+            __syncthreads();
+            at += w0 - mine + base;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (keep >> u & 1u) P.surv[hb + at++] = i0 + u * (int)blockDim.x + tid;
+        }
+    }
+    // The launch's last CTA plans the second pass.
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(&P.counters[kCPruned], 1ull) == gridDim.x - 1;
+    __syncthreads();
+    if (last) {
+        __threadfence();
+        score_plan(P, 1);
+    }
+    cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
 // ---------------------------------------------------------- candidates -----
@@ -1302,7 +1557,6 @@ __device__ __forceinline__ unsigned long long cand_key(float s, float t, float i
 
 __global__ void k_select(Pools P) {
     __shared__ float thr[kMaxRoundsPerStep], inv_safe[kMaxRoundsPerStep];
-    __shared__ int rh[kMaxRoundsPerStep];
     __shared__ unsigned hist[256];
     __shared__ int cnt0, fill, mode, drop_safe;
     __shared__ unsigned need;
@@ -1325,22 +1579,21 @@ __global__ void k_select(Pools P) {
         fill = 0;
         drop_safe = 0;
     }
-    for (int r = threadIdx.x; r < kMaxRoundsPerStep; r += blockDim.x) rh[r] = 0;
     __syncthreads();
-    const int nh = f.hyp_count;
     const int64_t hb = f.hyp_base;
+    // The hypotheses with a full score: all, or those k_prune left.
+    const int32_t *list = f.m_blocks ? P.surv + hb : nullptr;
+    const int nh = list ? f.surv : f.hyp_count;
     int my = 0;
-    for (int i = threadIdx.x; i < nh; i += blockDim.x) {
+    for (int j = threadIdx.x; j < nh; j += blockDim.x) {
+        const int i = list ? list[j] : j;
         const float s = P.hS32[hb + i];
-        const int64_t r = ((P.hId[hb + i] >> 2) - f.step_first) / f.step_div;
-        const float pm = thr[r];
-        atomicAdd(&rh[r], 1);
+        const float pm = thr[round_of(f, P.hId[hb + i])];
         my += (s <= pm + (pm * (1.0f / 4096.0f) + 1.0f)) ? 1 : 0;
     }
     my = warp_sum(my);
     if ((threadIdx.x & 31) == 0) atomicAdd(&cnt0, my);
     __syncthreads();
-    for (int r = threadIdx.x; r < kMaxRoundsPerStep; r += blockDim.x) f.round_hyps[r] = rh[r];
     if (threadIdx.x == 0) {
         const bool forced = f.force_samples > 0;
         const bool splittable = forced ? f.step_samples > kSplitSamples : f.step_rounds > 1;
@@ -1396,10 +1649,11 @@ __global__ void k_select(Pools P) {
             const unsigned long long hi_mask = pass == 0 ? 0ull : (~0ull << (shift + 8));
             for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
             __syncthreads();
-            for (int i = threadIdx.x; i < nh; i += blockDim.x) {
+            for (int j = threadIdx.x; j < nh; j += blockDim.x) {
+                const int i = list ? list[j] : j;
                 const float s = P.hS32[hb + i];
                 const int64_t id = P.hId[hb + i];
-                const int64_t r = ((id >> 2) - f.step_first) / f.step_div;
+                const int r = round_of(f, id);
                 const float pm = thr[r];
                 if (!(s <= pm + (pm * (1.0f / 4096.0f) + 1.0f))) continue;
                 const unsigned long long key = cand_key(s, pm, inv_safe[r], id, f.step_first);
@@ -1422,10 +1676,11 @@ __global__ void k_select(Pools P) {
     }
     const unsigned long long kmax = mode == 1 ? kstar : ~0ull;
     const int cap = f.cand_count;
-    for (int i = threadIdx.x; i < nh; i += blockDim.x) {
+    for (int j = threadIdx.x; j < nh; j += blockDim.x) {
+        const int i = list ? list[j] : j;
         const float s = P.hS32[hb + i];
         const int64_t id = P.hId[hb + i];
-        const int64_t r = ((id >> 2) - f.step_first) / f.step_div;
+        const int r = round_of(f, id);
         const float pm = thr[r];
         if (!(s <= pm + (pm * (1.0f / 4096.0f) + 1.0f))) continue;
         if (mode == 1) {
@@ -1609,55 +1864,69 @@ __global__ void __launch_bounds__(256) k_finalize(Pools P) {
     const int C = f.cand_count;
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
         const int64_t id = P.hId[f.hyp_base + P.cHyp[f.cand_base + c]];
-        const int64_t r = ((id >> 2) - f.step_first) / f.step_div;
+        const int r = round_of(f, id);
         atomicMin(&rmin[r], dbl_to_ordered(P.cS64[f.cand_base + c]));
     }
     __syncthreads();
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
         const int64_t id = P.hId[f.hyp_base + P.cHyp[f.cand_base + c]];
-        const int64_t r = ((id >> 2) - f.step_first) / f.step_div;
+        const int r = round_of(f, id);
         if (dbl_to_ordered(P.cS64[f.cand_base + c]) == rmin[r]) atomicMin(&rid[r], (unsigned long long)id);
     }
     __syncthreads();
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
         const int64_t id = P.hId[f.hyp_base + P.cHyp[f.cand_base + c]];
-        const int64_t r = ((id >> 2) - f.step_first) / f.step_div;
+        const int r = round_of(f, id);
         if ((unsigned long long)id == rid[r]) rwin[r] = c;
+    }
+    __shared__ int64_t s_end;
+    __shared__ int hyps;
+    __syncthreads();
+    const bool forced = f.force_samples > 0;
+    bool stop = false;
+    if (threadIdx.x == 0) {
+        f.rescored += C;
+        int64_t r_end = f.step_rounds;
+        for (int64_t r = 0; r < f.step_rounds; ++r) {
+            const int c = rwin[r];
+            if (c >= 0) {
+                const int64_t cs = f.cand_base + c;
+                const double bs = P.cS64[cs];
+                if (!f.found || bs < f.best_score) {
+                    const int64_t bid = (int64_t)rid[r];
+                    f.found = 1;
+                    f.best_score = bs;
+                    f.best_count = P.cCnt[cs];
+                    f.best_sample = bid >> 2;
+                    f.best_sol = (int32_t)(bid & 3);
+                    const double *Pp = P.hP64 + 12 * (f.hyp_base + P.cHyp[cs]);
+                    for (int e = 0; e < 12; ++e) f.best_P[e] = Pp[e];
+                }
+            }
+            if (forced) continue;
+            const int64_t after = f.step_first + (r + 1) * f.B;
+            const int64_t need = needed_samples(f.found ? f.best_count : 0, f.n, f.log_missing, f.trials_mult, f.quirk);
+            if ((after > need && after >= f.min_samples) || after >= f.max_total) {
+                stop = true;
+                r_end = r + 1;
+                break;
+            }
+        }
+        s_end = r_end;
+        hyps = r_end == f.step_rounds ? f.hyp_count : 0;
+    }
+    __syncthreads();
+    // Hypotheses of the rounds actually consumed.
+    const int64_t r_end = s_end;
+    if (r_end < f.step_rounds) {
+        const int64_t end_id = 4 * (f.step_first + r_end * f.B);
+        int mine = 0;
+        for (int i = threadIdx.x; i < f.hyp_count; i += blockDim.x) mine += P.hId[f.hyp_base + i] < end_id ? 1 : 0;
+        mine = warp_sum(mine);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&hyps, mine);
     }
     __syncthreads();
     if (threadIdx.x != 0) return;
-    f.rescored += C;
-    const bool forced = f.force_samples > 0;
-    bool stop = false;
-    int64_t r_end = f.step_rounds;
-    for (int64_t r = 0; r < f.step_rounds; ++r) {
-        const int c = rwin[r];
-        if (c >= 0) {
-            const int64_t cs = f.cand_base + c;
-            const double bs = P.cS64[cs];
-            if (!f.found || bs < f.best_score) {
-                const int64_t bid = (int64_t)rid[r];
-                f.found = 1;
-                f.best_score = bs;
-                f.best_count = P.cCnt[cs];
-                f.best_sample = bid >> 2;
-                f.best_sol = (int32_t)(bid & 3);
-                const double *Pp = P.hP64 + 12 * (f.hyp_base + P.cHyp[cs]);
-                for (int e = 0; e < 12; ++e) f.best_P[e] = Pp[e];
-            }
-        }
-        if (forced) continue;
-        const int64_t after = f.step_first + (r + 1) * f.B;
-        const int64_t need = needed_samples(f.found ? f.best_count : 0, f.n, f.log_missing, f.trials_mult, f.quirk);
-        if ((after > need && after >= f.min_samples) || after >= f.max_total) {
-            stop = true;
-            r_end = r + 1;
-            break;
-        }
-    }
-    // Hypotheses of the rounds actually consumed.
-    int64_t hyps = 0;
-    for (int64_t r = 0; r < r_end; ++r) hyps += f.round_hyps[r];
     f.hyps_done += hyps;
     f.steps += 1;
     if (forced) {
