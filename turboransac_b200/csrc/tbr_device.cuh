@@ -428,22 +428,23 @@ __device__ __forceinline__ void quat_rotate(const double *q, double p1, double p
     out[2] = px3 * q2 - px2 * q3 - px1 * q4 + px4 * q1;
 }
 
-// q <- q * exp(w) (quat_step_post with quat_exp's Taylor branch, pose_utils.cuh:138-188).
+// q <- q * exp(w) (quat_step_post with quat_exp, pose_utils.cuh:138-188). For
+// angles below 1/2 the half-angle cosine and sinc are their Taylor polynomials in
+// theta^2 (terms to theta^14, remainder below 1e-19), without the square
+// root, sine and cosine on the serial path of an LM iteration.
 __device__ __forceinline__ void quat_step_post(const double *q, const double *w, double *out) {
-    const double theta2 = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
-    const double theta = sqrt(theta2);
-    const double th = 0.5 * theta;
-    double re, im;
-    if (theta > 1e-6) {
+    const double u = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
+    double re, im;  // cos(theta / 2), sin(theta / 2) / theta
+    if (u < 0.25) {
+        const double h = 0.25 * u;  // (theta / 2)^2
+        re = 1.0 + h * (-1.0 / 2 + h * (1.0 / 24 + h * (-1.0 / 720 + h * (1.0 / 40320 + h * (-1.0 / 3628800 +
+             h * (1.0 / 479001600 + h * (-1.0 / 87178291200.0)))))));
+        im = 0.5 + 0.5 * h * (-1.0 / 6 + h * (1.0 / 120 + h * (-1.0 / 5040 + h * (1.0 / 362880 + h * (-1.0 / 39916800 +
+             h * (1.0 / 6227020800.0 + h * (-1.0 / 1307674368000.0)))))));
+    } else {
+        const double theta = sqrt(u), th = 0.5 * theta;
         re = cos(th);
         im = sin(th) / theta;
-    } else {
-        const double theta4 = theta2 * theta2;
-        re = 1.0 - (1.0 / 8.0) * theta2 + (1.0 / 384.0) * theta4;
-        im = 0.5 - (1.0 / 48.0) * theta2 + (1.0 / 3840.0) * theta4;
-        const double s = sqrt(re * re + im * im * theta2);
-        re /= s;
-        im /= s;
     }
     const double b[4] = {re, im * w[0], im * w[1], im * w[2]};
     out[0] = q[0] * b[0] - q[1] * b[1] - q[2] * b[2] - q[3] * b[3];
@@ -475,6 +476,17 @@ __device__ __forceinline__ uint64_t f2mul(uint64_t a, uint64_t b) {
 __device__ __forceinline__ uint64_t f2add(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// (without flushing denormals, as scalar code)
+__device__ __forceinline__ uint64_t f2add_rn(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t f2sub(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 // rn(a*b + c) clamped to [0, 1] (NaN becomes 0).

@@ -2023,110 +2023,159 @@ __global__ void __launch_bounds__(1024) k_inliers(Pools P) {
 }
 
 // ------------------------------------------------------------------ LM -----
-__device__ __forceinline__ void kahan_add(float &s, float &c, float x) {
-    const float y = x - c;
-    const float t = s + y;
-    c = (t - s) - y;
-    s = t;
-}
-
-// Block-wide FP64 sum of NV values per thread; every thread gets the result in
-// out[] (shared). Uses 32*NV doubles of scratch.
-template <int NV>
-__device__ __forceinline__ void block_sum_d(double (&v)[NV], double *scratch, double *out) {
-    static_assert(NV <= 32, "one value per lane after the warp reduction");
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // Warp reduce-scatter by recursive halving: at width h a lane trades the
-    // half of its 2h partial sums that its partner (lane ^ h) keeps, so after
-    // 16 + 8 + 4 + 2 + 1 exchanges lane k holds the warp's sum of value k.
-    double a[32];
-#pragma unroll
-    for (int k = 0; k < 32; ++k) a[k] = k < NV ? v[k] : 0.0;
-#pragma unroll
-    for (int h = 16; h >= 1; h >>= 1) {
-        const bool upper = (lane & h) != 0;
-#pragma unroll
-        for (int k = 0; k < h; ++k) {
-            const double keep = upper ? a[k + h] : a[k];
-            const double give = upper ? a[k] : a[k + h];
-            a[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
-        }
-    }
-    if (lane < NV) scratch[w * NV + lane] = a[0];
-    __syncthreads();
-    if (threadIdx.x < NV) {
-        double s = 0.0;
-        for (int q = 0; q < nw; ++q) s += scratch[q * NV + threadIdx.x];
-        out[threadIdx.x] = s;
-    }
-    __syncthreads();
-}
-
 constexpr int kLMCluster = 8;  // CTAs cooperating on one frame's LM
 
-constexpr int kLMSums = 28;  // cost + 21 J^T W J + 6 J^T W r
+constexpr int kLMSums = 28;  // 21 J^T W J, 6 J^T W r, cost
 enum LMLoss : int32_t { kLossCauchy = 0, kLossTruncated = 1, kLossHuber = 2, kLossTrivial = 3 };
 
-// One pass over inliers [i0, i1) at pose (q, t): the FP64 Cauchy cost
+__device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+
+// Two compensated FP32 sums (S - C, S the rounded sum, C its excess) added to two
+// others in place (packed FP32x2): the rounding error of S + S2 (Knuth's
+// TwoSum) goes into C.
+__device__ __forceinline__ void pair_add2(uint64_t &S, uint64_t &C, uint64_t S2, uint64_t C2) {
+    const uint64_t t = f2add_rn(S, S2), b = f2sub(t, S);
+    const uint64_t e = f2add_rn(f2sub(S, f2sub(t, b)), f2sub(S2, b));
+    C = f2sub(f2add_rn(C, C2), e);
+    S = t;
+}
+
+// Sum over the warp of 28 compensated FP32 sums per lane, in pairs: lane k returns
+// the sum of value k in FP64. Reduce-scatter by recursive halving: a lane trades the
+// half of its pairs that its partner keeps (8 + 4 + 2 + 1 pairs at distances 16, 8,
+// 4, 2), then one value of the last pair at distance 1. In FP32 pairs, since
+// converting 56 values a lane to FP64 first takes longer than the whole reduction.
+__device__ __forceinline__ double warp_scatter_pairs(const uint64_t (&S)[14], const uint64_t (&C)[14]) {
+    const int lane = threadIdx.x & 31;
+    uint64_t s[16], c[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) s[k] = k < 14 ? S[k] : 0ull, c[k] = k < 14 ? C[k] : 0ull;
+#pragma unroll
+    for (int h = 8; h >= 1; h >>= 1) {
+        const bool upper = (lane & (2 * h)) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            if (k + h >= 14 && k >= 14) continue;
+            const uint64_t gs = shfl_xor64(upper ? s[k] : s[k + h], 2 * h);
+            const uint64_t gc = shfl_xor64(upper ? c[k] : c[k + h], 2 * h);
+            s[k] = upper ? s[k + h] : s[k];
+            c[k] = upper ? c[k + h] : c[k];
+            pair_add2(s[k], c[k], gs, gc);
+        }
+    }
+    float s0, s1, c0, c1;
+    f2unpack(s[0], s0, s1);
+    f2unpack(c[0], c0, c1);
+    const bool odd = (lane & 1) != 0;
+    const float gs = __shfl_xor_sync(0xffffffffu, odd ? s0 : s1, 1), gc = __shfl_xor_sync(0xffffffffu, odd ? c0 : c1, 1);
+    return ((double)(odd ? s1 : s0) - (double)(odd ? c1 : c0)) + ((double)gs - (double)gc);
+}
+
+// What the LM evaluates: the camera and loss of a frame.
+struct LMModel {
+    double fx, fy, cx, cy, inv_sq, thr;
+    int loss;
+    bool weighted;
+    float fxf, fyf, isqf;  // fx, fy, inv_sq
+};
+
+// Kahan step of two accumulators at once (packed FP32x2): S += x, C the carried error.
+__device__ __forceinline__ void kahan_add2(uint64_t &S, uint64_t &C, uint64_t x) {
+    const uint64_t y = f2sub(x, C), t = f2add_rn(S, y);
+    C = f2sub(f2sub(t, S), y);
+    S = t;
+}
+
+// One pass over inliers [i0, i1) at the pose R, t (12 doubles): the FP64 cost
 // (jaco.cuh:31-104) and, from the same FP64 residuals, the J^T W J lower
 // triangle (jaco.cuh:173-200) and J^T W r (:202-209) accumulated in FP32 with
-// Kahan compensation. The Jacobian uses the world coordinates of the
-// reference's parameterisation (rotation post-multiplied, translation t + R dt).
-// out[0] = cost, out[1..27] = accumulators (block totals).
-__device__ void lm_pass(const Pools &P, int64_t base, int64_t i0, int64_t i1, const double *q, const double *t,
-                        const double *cam, double inv_sq_thr, int loss, double thr, bool weighted,
-                        double *scratch, double *out) {
-    double R[9];
-    quat_to_rotmat(q, R);
-    const float r00 = (float)R[0], r01 = (float)R[1], r02 = (float)R[2], r10 = (float)R[3], r11 = (float)R[4],
-                r12 = (float)R[5], r20 = (float)R[6], r21 = (float)R[7], r22 = (float)R[8];
-    const float fx = (float)cam[0], fy = (float)cam[1];
-    const float isq = (float)inv_sq_thr;
-    double cost = 0.0;
-    float Sv[27], Cc[27];
+// Kahan compensation, in the reference's parameterisation (rotation
+// post-multiplied, translation t + R dt). Each warp leaves its 28 sums in
+// scratch[warp]; the number of warps with points is returned.
+//
+// The FP32 rounding of J^T W r decides where the LM comes to rest (about 1e-10
+// from the FP64 optimum), so its terms keep their form; the rest is arranged for
+// few instructions on a short chain: the Cauchy cost, sum log(1 + a), a = r^2 /
+// s^2, is taken as one log1p a thread, of the product of the 1 + a kept as q =
+// product - 1 (exact to rounding for small a); the Kahan sums run two to a packed
+// instruction and stay FP32 pairs in the warp's reduction. What bounds it is the
+// latency of one point's FP64 and FP32 chain (about 1400 cycles, two points in
+// flight) and of the reduction (about 1300).
+template <bool kCauchy>
+__device__ __forceinline__ int lm_pass(const Pools &P, int64_t base, int i0, int i1, const double *pose,
+                                       const float *Rf, const LMModel &m, double (*scratch)[kLMSums]) {
+    double R[9], t[3];
 #pragma unroll
-    for (int k = 0; k < 27; ++k) Sv[k] = Cc[k] = 0.0f;
-#pragma unroll 2  // two points per thread in flight: the FP64 division and log1p chains overlap
-    for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    for (int k = 0; k < 9; ++k) R[k] = pose[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t[k] = pose[9 + k];
+    const float r00 = Rf[0], r01 = Rf[1], r02 = Rf[2], r10 = Rf[3], r11 = Rf[4], r12 = Rf[5], r20 = Rf[6],
+                r21 = Rf[7], r22 = Rf[8];
+    const float fx = m.fxf, fy = m.fyf, isq = m.isqf;
+    double cost = 0.0, q = 0.0;
+    uint64_t S[14], C[14];
+#pragma unroll
+    for (int k = 0; k < 14; ++k) S[k] = C[k] = 0ull;
+#pragma unroll 2
+    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
         const int64_t o = base + i;
         const double X0d = P.lX64[3 * o], X1d = P.lX64[3 * o + 1], X2d = P.lX64[3 * o + 2];
+        const double u = P.lx64[2 * o], v = P.lx64[2 * o + 1];
         const double Z0 = R[0] * X0d + R[1] * X1d + R[2] * X2d + t[0];
         const double Z1 = R[3] * X0d + R[4] * X1d + R[5] * X2d + t[1];
         const double Z2 = R[6] * X0d + R[7] * X1d + R[8] * X2d + t[2];
         const bool valid = Z2 >= 0.0;
-        const double inv_z = 1.0 / Z2;
-        const double z0d = Z0 * inv_z, z1d = Z1 * inv_z;
-        const double r0 = (cam[0] * z0d + cam[2]) - P.lx64[2 * o];
-        const double r1 = (cam[1] * z1d + cam[3]) - P.lx64[2 * o + 1];
-        const double r_squared = r0 * r0 + r1 * r1;
+        double inv_z, r0, r1, r_squared;
+        double lc = 0.0, a = 0.0;
+        if (kCauchy) {
+            inv_z = 1.0 / Z2;
+            r0 = (m.fx * (Z0 * inv_z) + m.cx) - u;
+            r1 = (m.fy * (Z1 * inv_z) + m.cy) - v;
+            r_squared = r0 * r0 + r1 * r1;
+            a = r_squared * m.inv_sq;
+        } else {
+            inv_z = 1.0 / Z2;
+            r0 = (m.fx * (Z0 * inv_z) + m.cx) - u;
+            r1 = (m.fy * (Z1 * inv_z) + m.cy) - v;
+            r_squared = r0 * r0 + r1 * r1;
+        }
         // FP32 Jacobian from the FP64 projection and residual.
-        const float iz = (float)inv_z, z0 = (float)z0d, z1 = (float)z1d;
+        const float iz = (float)inv_z, z0 = (float)(Z0 * inv_z), z1 = (float)(Z1 * inv_z);
         const float rx = (float)r0, ry = (float)r1;
         const float r2 = (float)r_squared;
         float wgt;
-        double lc;
-        if (loss == kLossCauchy) {  // CauchyLoss_cuda, robust_loss.cuh:24-38
-            lc = log1p(r_squared * inv_sq_thr);
+        if (kCauchy || m.loss == kLossCauchy) {  // CauchyLoss_cuda, robust_loss.cuh:24-38
+            if (!kCauchy) lc = log1p(r_squared * m.inv_sq);
             wgt = fmaxf(isq / (1.0f + r2 * isq), FLT_MIN);
         } else {
-            const double sq = thr * thr;
-            if (loss == kLossTruncated) {  // TruncatedLoss_cuda, robust_loss.cuh:10-22
+            const double sq = m.thr * m.thr;
+            if (m.loss == kLossTruncated) {  // TruncatedLoss_cuda, robust_loss.cuh:10-22
                 lc = fmin(r_squared, sq);
                 wgt = r_squared < sq ? 1.0f : 0.0f;
-            } else if (loss == kLossHuber) {
-                lc = r_squared <= sq ? r_squared : 2.0 * thr * sqrt(r_squared) - sq;
-                wgt = r_squared <= sq ? 1.0f : (float)(thr / sqrt(r_squared));
+            } else if (m.loss == kLossHuber) {
+                lc = r_squared <= sq ? r_squared : 2.0 * m.thr * sqrt(r_squared) - sq;
+                wgt = r_squared <= sq ? 1.0f : (float)(m.thr / sqrt(r_squared));
             } else {
                 lc = r_squared;
                 wgt = 1.0f;
             }
         }
-        if (weighted) {
-            const double m = P.lw64[o];
-            lc *= m;
-            wgt *= (float)m;
+        if (!kCauchy && m.weighted) {
+            const double mult = P.lw64[o];
+            lc *= mult;
+            wgt *= (float)mult;
         }
-        cost += valid ? lc : 0.0;
+        if (kCauchy) {
+            a = valid ? a : 0.0;
+            if (q > 0x1p100 || a > 0x1p100) {  // (kept far from overflow)
+                cost += log1p(q) + log1p(a);
+                q = 0.0;
+            } else {
+                q = fma(q, a, q + a);
+            }
+        } else {
+            cost += valid ? lc : 0.0;
+        }
         const float wv = valid ? wgt : 0.0f;
         const float a0 = fx * iz, a2 = -fx * z0 * iz;
         const float b1 = fy * iz, b2 = -fy * z1 * iz;
@@ -2140,7 +2189,7 @@ __device__ void lm_pass(const Pools &P, int64_t base, int64_t i0, int64_t i1, co
         const float d22 = wv * (dZ02 * dZ02 + dZ12 * dZ12);
         const float X0 = (float)X0d, X1 = (float)X1d, X2 = (float)X2d;
         const float wx = wv * rx, wy = wv * ry;
-        const float v[27] = {
+        const float val[28] = {
             X2 * (X2 * d11 - X1 * d21) + X1 * (X1 * d22 - X2 * d21),
             -X2 * (X2 * d10 - X0 * d21) - X1 * (X0 * d22 - X2 * d20),
             X1 * (X0 * d21 - X1 * d20) - X2 * (X0 * d11 - X1 * d10),
@@ -2162,43 +2211,61 @@ __device__ void lm_pass(const Pools &P, int64_t base, int64_t i0, int64_t i1, co
             wx * (X0 * dZ01 - X1 * dZ00) + wy * (X0 * dZ11 - X1 * dZ10),
             dZ00 * wx + dZ10 * wy,
             dZ01 * wx + dZ11 * wy,
-            dZ02 * wx + dZ12 * wy};
+            dZ02 * wx + dZ12 * wy,
+            0.0f};
 #pragma unroll
-        for (int k = 0; k < 27; ++k) kahan_add(Sv[k], Cc[k], v[k]);
+        for (int k = 0; k < 14; ++k) kahan_add2(S[k], C[k], f2pack(val[2 * k], val[2 * k + 1]));
     }
-    double dv[kLMSums];
-    dv[0] = cost;
+    const int nw = min((int)(blockDim.x >> 5), (i1 - i0 + 31) >> 5);
+    const int warp = threadIdx.x >> 5;
+    if (warp < nw) {
+        // Lanes 0 to 26: the accumulators; the cost (any lane's) goes to place 27.
+        const int lane = threadIdx.x & 31;
+        double s = warp_scatter_pairs(S, C);
+        if (kCauchy) cost += log1p(q);
 #pragma unroll
-    for (int k = 0; k < 27; ++k) dv[1 + k] = (double)Sv[k] - (double)Cc[k];
-    block_sum_d<kLMSums>(dv, scratch, out);
+        for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
+        if (lane == kLMSums - 1) s = cost;
+        if (lane < kLMSums) scratch[warp][lane] = s;
+    }
+    return nw;
 }
 
-// 6x6 Cholesky solve of the damped normal equations (lm_utils.cuh:14-100),
-// non-positive pivots replaced by 1e-15 as there, with reciprocal pivots.
-__device__ __forceinline__ void cholesky_solve6(const double *A, const double *b, double *x) {
-    double L[36], inv[6], y[6];
-    for (int i = 0; i < 6; ++i)
-        for (int j = 0; j <= i; ++j) {
-            double sum = 0.0;
-            for (int k = 0; k < j; ++k) sum += L[i * 6 + k] * L[j * 6 + k];
-            if (i == j) {
-                double val = A[i * 6 + i] - sum;
-                if (val <= 0.0) val = 1e-15;
-                L[i * 6 + i] = sqrt(val);
-                inv[i] = 1.0 / L[i * 6 + i];
-            } else {
-                L[i * 6 + j] = (A[i * 6 + j] - sum) * inv[j];
-            }
+// The damped normal equations (lm_utils.cuh:14-100): Cholesky of the lower
+// triangle H (21, column by column) + lambda I, non-positive pivots replaced by
+// 1e-15 as there, with the reciprocal pivots taken as reciprocal square roots;
+// x = (H + lambda I)^-1 g.
+__device__ __forceinline__ void cholesky_solve6(const double *H, double lambda, const double *g, double (&x)[6]) {
+    double L[6][6], inv[6], y[6];
+    int k = 0;
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+#pragma unroll
+        for (int r = c; r < 6; ++r) L[r][c] = H[k++] + (r == c ? lambda : 0.0);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) y[c] = g[c];
+    // Right-looking: each column's updates are independent of one another; the
+    // right-hand side rides along as a seventh row.
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        double d = L[c][c];
+        if (d <= 0.0) d = 1e-15;
+        inv[c] = rsqrt(d);
+        y[c] *= inv[c];
+#pragma unroll
+        for (int r = c + 1; r < 6; ++r) L[r][c] *= inv[c];
+#pragma unroll
+        for (int r = c + 1; r < 6; ++r) {
+            y[r] -= L[r][c] * y[c];
+#pragma unroll
+            for (int q = c + 1; q <= r; ++q) L[r][q] -= L[r][c] * L[q][c];
         }
-    for (int i = 0; i < 6; ++i) {
-        double sum = 0.0;
-        for (int j = 0; j < i; ++j) sum += L[i * 6 + j] * y[j];
-        y[i] = (b[i] - sum) * inv[i];
     }
-    for (int i = 5; i >= 0; --i) {
-        double sum = 0.0;
-        for (int j = i + 1; j < 6; ++j) sum += L[j * 6 + i] * x[j];
-        x[i] = (y[i] - sum) * inv[i];
+#pragma unroll
+    for (int c = 5; c >= 0; --c) {
+        x[c] = y[c] * inv[c];
+#pragma unroll
+        for (int r = 0; r < c; ++r) y[r] -= L[c][r] * x[c];
     }
 }
 
@@ -2206,142 +2273,127 @@ __device__ __forceinline__ void cholesky_solve6(const double *A, const double *b
 // accept rule, the lambda schedule, the removal of damping after a rejected
 // step, and both stop tests -- one frame per cluster of CL CTAs, each owning a
 // slice of the inliers. Every candidate pose gets one fused pass (cost and, for
-// the case it is accepted, the normal equations at it), so an iteration costs
-// one pass and two cluster barriers. Sums cross the block and cluster in FP64 in
-// a fixed order; the solve, the step and the acceptance test are FP64.
+// the case it is accepted, the normal equations at it). Sums cross the warps,
+// the CTA and the cluster in FP64 in a fixed order; then warp 0 of every CTA
+// accepts or rejects and solves for the next candidate, each for itself and all
+// alike, so an iteration costs one pass, two CTA barriers and, in a cluster,
+// one cluster barrier. Measured cycles an iteration (pass, sums, solve), before
+// -> now: 799 inliers on one CTA 12000 -> 9000 (6500 + 500 + 2000), 13986 on 8 CTAs
+// 26500 -> 15700 (12000 + 1800 + 1900); the LM of the 256-frame batch 0.9 -> 0.55 ms.
 template <int CL>
 __device__ __forceinline__ void lm_frame(const Pools &P, int slot) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    __shared__ double scratch[32 * kLMSums];
-    __shared__ double part[kLMSums];  // this CTA's pass totals
-    __shared__ double tot[kLMSums];   // rank 0: cluster totals
-    __shared__ double J[36], g[6], Jc[28], q[4], t[3], qn[4], tn[3];
+    __shared__ double scratch[kLMSmallThreads / 32][kLMSums];
+    __shared__ double part[2][CL][kLMSums];  // CTA totals of the pass, by its parity
+    __shared__ double T[kLMSums], H[kLMSums];  // the pass's totals; those at the current pose
+    __shared__ double q[4], t[3], qn[4];       // current pose; candidate
+    __shared__ double pose[12];                // R, t of the candidate
+    __shared__ float poseR[9];                 // R in FP32
     __shared__ double cost, lambda;
-    __shared__ int brk, recompute, iters, invalid;
-    __shared__ double pq[4], pt[3];  // the pose every CTA evaluates next
-    __shared__ int pbrk;
+    __shared__ int stop, iters, invalid;
     const int rank = (int)cluster.block_rank();
+    const int lane = threadIdx.x & 31;
     FrameDev &f = P.frames[slot];
     FrameResult &res = P.results[slot];
     const int64_t base = f.blk_off * kSub;
     const int64_t n = f.num_inliers;
-    const int64_t i0 = n * rank / CL, i1 = n * (rank + 1) / CL;
-    const double cam[4] = {f.lm_cam[0], f.lm_cam[1], f.lm_cam[2], f.lm_cam[3]};
-    const double inv_sq_thr = f.lm_inv_sq_thr;
+    const int i0 = (int)(n * rank / CL), i1 = (int)(n * (rank + 1) / CL);
+    const LMModel m = {f.lm_cam[0], f.lm_cam[1], f.lm_cam[2], f.lm_cam[3], f.lm_inv_sq_thr, f.lm_thr,
+                       f.lm_loss,   f.lm_weighted != 0, (float)f.lm_cam[0], (float)f.lm_cam[1], (float)f.lm_inv_sq_thr};
+    const bool cauchy = m.loss == kLossCauchy && !m.weighted;
     const int64_t max_it = f.skip_refine ? 0 : f.lm_max_iter;
     // Read once: every barrier of the loop would reload them from the record.
     const double grad_tol = f.lm_grad_tol, step_tol = f.lm_step_tol, min_lambda = f.lm_min_lambda,
-                 max_lambda = f.lm_max_lambda, thr = f.lm_thr;
-    const int loss = f.lm_loss;
-    const bool weighted = f.lm_weighted != 0;
-
-    auto cluster_totals = [&]() {  // after lm_pass: every CTA's part -> rank 0's tot
-        cluster.sync();
-        if (rank == 0 && threadIdx.x < kLMSums) {
-            double acc = 0.0;
-            for (int r = 0; r < CL; ++r) acc += cluster.map_shared_rank(part, r)[threadIdx.x];
-            tot[threadIdx.x] = acc;
+                 max_lambda = f.lm_max_lambda;
+    if (threadIdx.x == 0) {
+        double R[9];
+        for (int k = 0; k < 4; ++k) q[k] = qn[k] = res.q[k];
+        for (int k = 0; k < 3; ++k) t[k] = pose[9 + k] = res.t[k];
+        quat_to_rotmat(q, R);
+        for (int k = 0; k < 9; ++k) pose[k] = R[k], poseR[k] = (float)R[k];
+        cost = 0.0;
+        lambda = f.lm_lambda0;
+        iters = invalid = 0;
+        stop = 0;
+    }
+    if constexpr (CL > 1) cluster.sync();  // every CTA runs before another writes its shared memory
+    else __syncthreads();
+    for (int64_t it = 0; max_it > 0; ++it) {
+        const int nw = cauchy ? lm_pass<true>(P, base, i0, i1, pose, poseR, m, scratch)
+                              : lm_pass<false>(P, base, i0, i1, pose, poseR, m, scratch);
+        __syncthreads();
+        if constexpr (CL > 1) {
+            if (threadIdx.x < kLMSums) {
+                double s = 0.0;
+                for (int k = 0; k < nw; ++k) s += scratch[k][lane];
+                for (int r = 0; r < CL; ++r) cluster.map_shared_rank(&part[it & 1][rank][0], r)[lane] = s;
+            }
+            cluster.sync();
+        }
+        if (threadIdx.x < 32) {
+            if (lane < kLMSums) {
+                double s = 0.0;
+                if constexpr (CL > 1)
+                    for (int k = 0; k < CL; ++k) s += part[it & 1][k][lane];
+                else
+                    for (int k = 0; k < nw; ++k) s += scratch[k][lane];
+                T[lane] = s;
+            }
+            __syncwarp();
+            const double c = T[kLMSums - 1];
+            const bool accept = it == 0 || c < cost;
+            if (accept && lane < kLMSums) H[lane] = T[lane];
+            __syncwarp();
+            if (lane == 0) {
+                if (it == 0) {
+                    cost = c;
+                    if (rank == 0) res.lm_cost0 = c;
+                } else {
+                    ++iters;
+                    if (accept) {
+                        for (int k = 0; k < 4; ++k) q[k] = qn[k];
+                        for (int k = 0; k < 3; ++k) t[k] = pose[9 + k];
+                        lambda = fmax(min_lambda, lambda / 10);
+                        cost = c;
+                    } else {
+                        ++invalid;
+                        lambda = fmin(max_lambda, lambda * 10);
+                    }
+                }
+                if (it >= max_it) {
+                    stop = 1;
+                } else {
+                    double x[6], gn = 0.0, sn = 0.0;
+                    cholesky_solve6(H, lambda, H + 21, x);
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) {
+                        x[k] = -x[k];
+                        gn += H[21 + k] * H[21 + k];
+                        sn += x[k] * x[k];
+                    }
+                    // lm.cuh:243-248 and the step test
+                    if (sqrt(gn) < grad_tol || sqrt(sn) < step_tol) {
+                        stop = 1;
+                    } else {
+                        double b[4], dt[3], R[9];
+                        quat_step_post(q, x, b);  // jaco.cuh:288-299
+                        quat_rotate(q, x[3], x[4], x[5], dt);
+                        quat_to_rotmat(b, R);
+                        for (int k = 0; k < 4; ++k) qn[k] = b[k];
+                        for (int k = 0; k < 9; ++k) pose[k] = R[k], poseR[k] = (float)R[k];
+                        for (int k = 0; k < 3; ++k) pose[9 + k] = t[k] + dt[k];
+                    }
+                }
+            }
         }
         __syncthreads();
-    };
-
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < 4; ++k) pq[k] = res.q[k];
-        for (int k = 0; k < 3; ++k) pt[k] = res.t[k];
-    }
-    __syncthreads();
-    if (max_it > 0)
-        lm_pass(P, base, i0, i1, pq, pt, cam, inv_sq_thr, loss, thr, weighted, scratch, part);
-    else if (threadIdx.x < kLMSums) part[threadIdx.x] = 0.0;
-    __syncthreads();
-    // One CTA: its pass totals are the frame's; a cluster sums its CTAs' in rank 0.
-    const double *T = CL == 1 ? part : tot;
-    if constexpr (CL > 1) cluster_totals();
-    if (rank == 0 && threadIdx.x == 0) {
-        for (int k = 0; k < 4; ++k) q[k] = pq[k];
-        for (int k = 0; k < 3; ++k) t[k] = pt[k];
-        cost = T[0];
-        for (int k = 0; k < 27; ++k) Jc[k] = T[1 + k];
-        Jc[27] = 0.0;
-        lambda = f.lm_lambda0;
-        recompute = 1;
-        iters = 0;
-        invalid = 0;
-        res.lm_cost0 = cost;
-    }
-    for (int64_t it = 0; it < max_it; ++it) {
-        if (rank == 0 && threadIdx.x == 0) {
-            brk = 0;
-            if (recompute) {
-                // J from the pass at the current pose (lower triangle in the
-                // reference's order); gradient test of lm.cuh:243-248.
-                const int idx[21][2] = {{0, 0}, {1, 0}, {2, 0}, {3, 0}, {4, 0}, {5, 0}, {1, 1},
-                                        {2, 1}, {3, 1}, {4, 1}, {5, 1}, {2, 2}, {3, 2}, {4, 2},
-                                        {5, 2}, {3, 3}, {4, 3}, {5, 3}, {4, 4}, {5, 4}, {5, 5}};
-                for (int k = 0; k < 36; ++k) J[k] = 0.0;
-                for (int k = 0; k < 21; ++k) J[idx[k][0] * 6 + idx[k][1]] = Jc[k];
-                double gn = 0.0;
-                for (int k = 0; k < 6; ++k) {
-                    g[k] = Jc[21 + k];
-                    gn += g[k] * g[k];
-                }
-                if (sqrt(gn) < grad_tol) brk = 1;
-            }
-            for (int k = 0; k < 6; ++k) J[k * 7] += lambda;
-            double x[6];
-            cholesky_solve6(J, g, x);
-            double sn = 0.0;
-            for (int k = 0; k < 6; ++k) {
-                x[k] = -1 * x[k];
-                sn += x[k] * x[k];
-            }
-            if (sqrt(sn) < step_tol) brk = 1;
-            quat_step_post(q, x, qn);  // jaco.cuh:288-299
-            double dt[3];
-            quat_rotate(q, x[3], x[4], x[5], dt);
-            for (int k = 0; k < 3; ++k) tn[k] = t[k] + dt[k];
-        }
-        if constexpr (CL == 1) {
-            // One CTA: the candidate pose and the stop flag are read in place;
-            // the pass's own barriers order this thread's next writes to them.
-            __syncthreads();
-            if (brk) break;
-            lm_pass(P, base, i0, i1, qn, tn, cam, inv_sq_thr, loss, thr, weighted, scratch, part);
-        } else {
-            cluster.sync();
-            if (threadIdx.x == 0) {
-                pbrk = cluster.map_shared_rank(&brk, 0)[0];
-                const double *rq = cluster.map_shared_rank(qn, 0), *rt = cluster.map_shared_rank(tn, 0);
-                for (int k = 0; k < 4; ++k) pq[k] = rq[k];
-                for (int k = 0; k < 3; ++k) pt[k] = rt[k];
-            }
-            __syncthreads();
-            if (pbrk) break;
-            lm_pass(P, base, i0, i1, pq, pt, cam, inv_sq_thr, loss, thr, weighted, scratch, part);
-            __syncthreads();
-            cluster_totals();
-        }
-        if (rank == 0 && threadIdx.x == 0) {
-            if (T[0] < cost) {
-                for (int k = 0; k < 4; ++k) q[k] = qn[k];
-                for (int k = 0; k < 3; ++k) t[k] = tn[k];
-                lambda = fmax(min_lambda, lambda / 10);
-                cost = T[0];
-                for (int k = 0; k < 27; ++k) Jc[k] = T[1 + k];
-                recompute = 1;
-            } else {
-                ++invalid;
-                for (int k = 0; k < 6; ++k) J[k * 7] -= lambda;
-                lambda = fmin(max_lambda, lambda * 10);
-                recompute = 0;
-            }
-            ++iters;
-        }
+        if (stop) break;
     }
     if (rank == 0 && threadIdx.x == 0) {
         for (int k = 0; k < 4; ++k) res.q[k] = q[k];
         for (int k = 0; k < 3; ++k) res.t[k] = t[k];
+        if (max_it <= 0) res.lm_cost0 = 0.0;
         res.lm_iters = iters;
         res.lm_invalid = invalid;
         res.lm_cost = cost;
@@ -2358,7 +2410,7 @@ __device__ __forceinline__ void lm_frame(const Pools &P, int slot) {
         res.overflow = f.overflow;
         res.status = kDone;
     }
-    cluster.sync();  // no CTA leaves while rank 0 may still read its shared memory
+    if constexpr (CL > 1) cluster.sync();  // no CTA leaves while another may still write its shared memory
     if (rank == 0 && threadIdx.x == 0) f.status = kDone;
 }
 
