@@ -545,7 +545,7 @@ class Engine {
     void launch_refine(const Pools &Q, int n_active, cudaStream_t st, Profile *prof = nullptr) {
         auto beg = [&](int k) { if (prof) cudaEventRecord(prof->ev[2 * k], st); };
         auto end = [&](int k) { if (prof) { cudaEventRecord(prof->ev[2 * k + 1], st); prof->launches[k]++; } };
-        beg(8); k_inliers<<<n_active, 1024, 0, st>>>(Q); end(8);
+        beg(8); k_inliers<<<n_active * kInlCtas, kInlThreads, 0, st>>>(Q); end(8);
         beg(9);
         // The one-CTA and the cluster LM take disjoint frames (by inlier
         // count): they run side by side, so the branch lasts as long as the
