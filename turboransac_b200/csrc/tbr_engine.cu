@@ -490,8 +490,8 @@ class Engine {
         bool armed = false;
     };
     static constexpr const char *kKernelNames[12] = {"k_plan", "k_sample_p3p", "k_score_plan", "k_score",
-                                                     "k_select", "k_rescore_plan", "k_rescore", "k_finalize",
-                                                     "k_inliers", "k_lm", "k_prune", "k_score"};
+                                                     "k_select", "k_prune", "k_rescore", "k_finalize",
+                                                     "k_inliers", "k_lm", "k_score"};
     // Scoring kernel variant: HR hypotheses per lane = 2*HP, PP points per iteration.
     void launch_score(const Pools &Q, int hr, int pp, cudaStream_t st, int pass = 0) {
         const int threads = kScoreWarps * 32;
@@ -523,7 +523,9 @@ class Engine {
     // The planning kernels are one CTA with a thread per frame (and 4 warps at least).
     static int plan_threads(int n_active) { return std::max(128, (n_active + 31) & ~31); }
     // RANSAC part of a step (plan .. finalize).
-    void launch_ransac(const Pools &Q, int n_active, int hr, cudaStream_t st, Profile *prof = nullptr) {
+    // With `loop` the step is a captured loop's body and ends it (k_finalize_loop).
+    void launch_ransac(const Pools &Q, int n_active, int hr, cudaStream_t st, Profile *prof = nullptr,
+                       const cudaGraphConditionalHandle *loop = nullptr) {
         auto beg = [&](int k) { if (prof) cudaEventRecord(prof->ev[2 * k], st); };
         auto end = [&](int k) { if (prof) { cudaEventRecord(prof->ev[2 * k + 1], st); prof->launches[k]++; } };
         beg(0); k_plan<<<1, plan_threads(n_active), 0, st>>>(Q); end(0);
@@ -533,13 +535,15 @@ class Engine {
         launch_score(Q, hr, pp, st);
         end(3);
         if (Q.prune) {  // second scoring pass, over what the first leaves
-            beg(10); launch_prune(Q, n_active, st); end(10);
-            beg(11); launch_score(Q, hr, pp, st, 1); end(11);
+            beg(5); launch_prune(Q, n_active, st); end(5);
+            beg(10); launch_score(Q, hr, pp, st, 1); end(10);
         }
         beg(4); k_select<<<n_active, 1024, 0, st>>>(Q); end(4);  // a frame's ~4000 hypotheses: 1024 threads (6.51 ms a batch, 256: 6.59)
-        beg(5); k_rescore_plan<<<1, plan_threads(n_active), 0, st>>>(Q); end(5);
         beg(6); k_rescore<<<rescore_grid, 256, 0, st>>>(Q); end(6);
-        beg(7); k_finalize<<<n_active, 256, 0, st>>>(Q); end(7);
+        beg(7);
+        if (loop) k_finalize_loop<<<n_active, 256, 0, st>>>(Q, *loop, 100000ull);
+        else k_finalize<<<n_active, 256, 0, st>>>(Q);
+        end(7);
     }
     // Refinement part: inliers + LM of frames whose RANSAC ended in an earlier step.
     void launch_refine(const Pools &Q, int n_active, cudaStream_t st, Profile *prof = nullptr) {
@@ -652,8 +656,7 @@ class Engine {
             ok = cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) ==
                  cudaSuccess;
             if (ok) {
-                launch_ransac(Q, n, hr, stream);
-                k_loop_ctl<<<1, 1, 0, stream>>>(Q, h, 100000ull);
+                launch_ransac(Q, n, hr, stream, nullptr, &h);
                 ok = cudaStreamEndCapture(stream, &body) == cudaSuccess;
             }
         }
@@ -738,10 +741,11 @@ class Engine {
             TBR_CUDA(cudaMemcpyAsync(h_counters, Q.counters, 8 * kCNum, cudaMemcpyDeviceToHost, stream));
             TBR_CUDA(cudaStreamSynchronize(stream));
             if (prof)
-                for (int k = 0; k < (Q.prune ? 12 : 10); ++k) {
+                for (int k = 0; k < 11; ++k) {
+                    if (!Q.prune && (k == 5 || k == 10)) continue;  // no second scoring pass
                     float ms = 0.f;
                     cudaEventElapsedTime(&ms, prof->ev[2 * k], prof->ev[2 * k + 1]);
-                    prof->ms[k == 11 ? 3 : k] += ms;  // both scoring passes together
+                    prof->ms[k == 10 ? 3 : k] += ms;  // both scoring passes together
                 }
             ++steps;
             if (h_counters[kCError] & kErrTimeout) return fail(TBR_ERR_TIMEOUT, "bounded device wait expired");
@@ -2310,7 +2314,7 @@ tbr_status tbr_batch_profile(tbr_batch *b, tbr_kernel_profile *out, int32_t max,
     if (st) return st;
     if (pairs_scored) *pairs_scored = E.h_counters[kCPairsTotal];
     int m = 0;
-    for (int k = 0; k < (b->Q.prune ? 11 : 10) && m < max; ++k, ++m) {
+    for (int k = 0; k < 10 && m < max; ++k, ++m) {
         std::snprintf(out[m].name, sizeof(out[m].name), "%s", Engine::kKernelNames[k]);
         out[m].total_ms = pr.ms[k];
         out[m].launches = pr.launches[k];

@@ -9,7 +9,7 @@
 //   k_prune         drops hypotheses that a random sample of the points rules out;
 //                   the rest are scored on the other points (a second pass)
 //   k_select        candidates within a safe band of each round's running minimum
-//   k_rescore_plan / k_rescore   exact FP64 MSAC of the candidates (reference formula)
+//   k_rescore       exact FP64 MSAC of the candidates (reference formula)
 //   k_finalize      the reference's selection and stop rule, round by round
 // then, for frames whose RANSAC ended:
 //   k_inliers       get_inliers_mx semantics + ordered compaction of the inliers
@@ -79,6 +79,9 @@ enum Counter : int {
     kCCandNext,
     kCTwoPass,  // pairs of the step's frames that are scored in two passes (0: none is)
     kCPruned,   // CTAs of k_prune that are done
+    kCSelected, // ... of k_select
+    kCFinal,    // ... of k_finalize
+    kCBlocks,   // hypothesis blocks of the first scoring pass (its arrival counters)
     kCSteps,
     kCPairsTotal,
     kCNum
@@ -210,6 +213,7 @@ struct Pools {
 // a usable model keeps sampling up to the sample cap.
 __device__ __forceinline__ int64_t needed_samples(int64_t inliers, int64_t n, double log_missing,
                                                   double mult, int quirk) {
+    if (inliers <= 0) return quirk ? (int64_t)INT_MIN : (int64_t)INT_MAX;  // log(1 - 0) = 0: an infinite bound
     const double w = (double)inliers / (double)n;
     const double prob_outlier = 1.0 - pow(w, 3.0);
     const double v = ceil(log_missing / log(prob_outlier) * mult);
@@ -217,7 +221,7 @@ __device__ __forceinline__ int64_t needed_samples(int64_t inliers, int64_t n, do
         if (!(v >= -2147483648.0 && v < 2147483648.0)) return (int64_t)INT_MIN;
         return (int64_t)(int)v;
     }
-    if (inliers <= 0 || !(v == v) || v >= 2147483647.0) return (int64_t)INT_MAX;
+    if (!(v == v) || v >= 2147483647.0) return (int64_t)INT_MAX;
     if (v <= -2147483648.0) return (int64_t)INT_MIN;
     return (int64_t)v;
 }
@@ -485,10 +489,15 @@ __global__ void k_plan(Pools P) {
                 r = max(r, (f->min_samples + f->B - 1) / f->B - f->rounds_done);
                 r = min(r, max_rounds - f->rounds_done);
                 r = min(r, (int64_t)(f->max_rounds_step > 0 ? f->max_rounds_step : kMaxRoundsPerStep));
-                // Growth cap: the frame's s-th step runs at most 4 * 2^(s-1) rounds,
-                // so a stop bound that shrinks once a better model turns up wastes
-                // at most the last step's overshoot.
-                if (f->steps >= 1) r = min(r, (int64_t)4 << min(f->steps - 1, 5));
+                // Growth cap: the frame's s-th step runs at most 8 * 2^(s-1) rounds (16 for
+                // small frames, whose rounds cost least), so a stop bound that shrinks
+                // once a better model turns up wastes at most the last step's overshoot.
+                // With 4 / 8 / 16 / 32 for all, device time of the steps: 256 frames 2.61
+                // / 2.57 / 2.62 / 2.91 ms, 160 served frames 2.18 / 2.19 / 2.36 / 2.89, one
+                // frame of 50000 points at 8 % inliers 796 / 751 / 805 / 890 us, of 20000
+                // at 15 % 427 / 350 / 363 / 366, of 5000 at 10 % 515 / 500 / 461 / 438, of 800
+                // at 12 % 359 / 311 / 267 / 315.
+                if (f->steps >= 1) r = min(r, (int64_t)(f->n < 8192 ? 16 : 8) << min(f->steps - 1, 4));
                 if (f->split > 0) r = min(r, (int64_t)f->split);
                 if (r < 1) r = 1;
                 rounds = r;
@@ -529,6 +538,8 @@ __global__ void k_plan(Pools P) {
         P.counters[kCCandNext] = 0;
         P.counters[kCTwoPass] = 0;
         P.counters[kCPruned] = 0;
+        P.counters[kCSelected] = 0;
+        P.counters[kCFinal] = 0;
         P.counters[kCStillRansac] = 0;
         P.counters[kCLMPending] = 0;
     }
@@ -554,11 +565,20 @@ struct P3PStage {  // one lane's sample, staged for its warp
     int a, n;       // active index of its frame, candidates
 };
 __global__ void __launch_bounds__(128) k_sample_p3p(Pools P) {
+    static_assert(kMaxRoundsPerStep <= 128, "a thread per round");
     __shared__ P3PStage stage[128];
     __shared__ int excl[128];
     const int64_t total = (int64_t)P.counters[kCSamplesTotal];
     const int lane = threadIdx.x & 31, wb = threadIdx.x & ~31;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    // For the scoring pass: round minima, and arrival counters of at most 4
+    // hypotheses a sample in blocks of 64 or more.
+    for (int k = blockIdx.x; k < P.n_active; k += gridDim.x) {
+        FrameDev &f = P.frames[P.active[k]];
+        if (threadIdx.x < f.step_rounds) f.round_min[threadIdx.x] = ~0ull;
+    }
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < min(total / 16 + P.n_active, P.max_hb); k += stride)
+        P.hb_arrive[k] = 0;
     for (int64_t g0 = (int64_t)blockIdx.x * blockDim.x; g0 < total; g0 += stride) {
         const int64_t g = g0 + threadIdx.x;
         const bool valid = g < total;
@@ -689,21 +709,23 @@ __device__ __forceinline__ int first_pass_blocks(const FrameDev &f) {
 // k_prune and the other points.
 __device__ __forceinline__ void score_plan(const Pools &P, int pass) {
     __shared__ int64_t sh[33];
-    __shared__ unsigned long long pairs_total;
+    __shared__ unsigned long long pairs_total, parts_total;
     const int a = threadIdx.x;
     FrameDev *f = a < P.n_active ? &P.frames[P.active[a]] : nullptr;
     bool act = f && f->step_samples > 0;
-    if (a == 0) pairs_total = 0;
+    if (a == 0) pairs_total = parts_total = 0;
     int hyps = 0, blocks = 0;  // of this pass
     __shared__ unsigned long long two_pass;  // pairs of the frames that could be scored in two passes
     if (pass == 0 && P.prune) {
         if (a == 0) two_pass = 0;
         __syncthreads();
+        unsigned long long tp = 0;
         if (act) {
             f->m_blocks = first_pass_blocks(*f);
-            if (f->m_blocks)
-                atomicAdd(&two_pass, (unsigned long long)f->hyp_count * (unsigned long long)f->n);
+            if (f->m_blocks) tp = (unsigned long long)f->hyp_count * (unsigned long long)f->n;
         }
+        tp = warp_sum(tp);
+        if ((a & 31) == 0 && tp) atomicAdd(&two_pass, tp);
         __syncthreads();
     }
     if (act) {
@@ -719,13 +741,14 @@ __device__ __forceinline__ void score_plan(const Pools &P, int pass) {
         }
     }
     __syncthreads();
+    unsigned long long pairs = 0, np = 0;
     if (act) {
         const int64_t n = pass ? f->n - (int64_t)f->m_blocks * kSub : min(f->n, (int64_t)blocks * kSub);
-        atomicAdd(&pairs_total, (unsigned long long)hyps * (unsigned long long)n);
+        pairs = (unsigned long long)hyps * (unsigned long long)n;
     }
+    pairs = warp_sum(pairs);
+    if ((a & 31) == 0 && pairs) atomicAdd(&pairs_total, pairs);
     __syncthreads();
-    __shared__ unsigned long long parts_total;
-    if (a == 0) parts_total = 0;
     int64_t items = 0, parts = 0, hbs = 0;
     int HB = 32, nhb = 0, cb = 1;
     if (act) {
@@ -748,8 +771,10 @@ __device__ __forceinline__ void score_plan(const Pools &P, int pass) {
         if (f->chunk_points > 0) cb = max(1, f->chunk_points / kSub);
         cb = max(cb, (blocks + kMaxScoreChunks - 1) / kMaxScoreChunks);
         cb = max(1, min(cb, blocks));
-        atomicAdd(&parts_total, (unsigned long long)hyps * ((blocks + cb - 1) / cb));
+        np = (unsigned long long)hyps * ((blocks + cb - 1) / cb);
     }
+    np = warp_sum(np);
+    if ((a & 31) == 0 && np) atomicAdd(&parts_total, np);
     __syncthreads();
     if (act) {
         // Keep the chunk partials within their buffer.
@@ -765,12 +790,6 @@ __device__ __forceinline__ void score_plan(const Pools &P, int pass) {
         items = (int64_t)nhb * nch;
         parts = (int64_t)hyps * nch;
         hbs = nhb;
-    }
-    // Round minima of every planned frame's rounds, reset a warp per frame.
-    for (int k = threadIdx.x >> 5; k < P.n_active; k += blockDim.x >> 5) {
-        FrameDev &g = P.frames[P.active[k]];
-        if (g.step_samples > 0 && (pass == 0 || g.m_blocks > 0))
-            for (int r = threadIdx.x & 31; r < (int)g.step_rounds; r += 32) g.round_min[r] = ~0ull;
     }
     int64_t tot;
     const int64_t iexcl = block_exclusive_scan(items, sh, tot);
@@ -788,9 +807,10 @@ __device__ __forceinline__ void score_plan(const Pools &P, int pass) {
     if (a == 0 && tot > P.max_parts) flag_error(P, kErrOverflow);
     const int64_t hexcl = block_exclusive_scan(hbs, sh, tot);
     if (act) f->hb_base = hexcl;
-    // The step's hypothesis-block arrival counters are [0, tot): zeroed by the block.
-    for (int64_t i = threadIdx.x; i < min(tot, P.max_hb); i += blockDim.x) P.hb_arrive[i] = 0;
-    if (a == 0 && tot > P.max_hb) flag_error(P, kErrOverflow);
+    if (a == 0) {
+        if (pass == 0) P.counters[kCBlocks] = (unsigned long long)min(tot, P.max_hb);
+        if (tot > P.max_hb) flag_error(P, kErrOverflow);
+    }
 }
 __global__ void k_score_plan(Pools P, int pass) { score_plan(P, pass); }
 
@@ -1406,10 +1426,12 @@ __global__ void __launch_bounds__(1024) k_prune(Pools P) {
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ float cut[kMaxRoundsPerStep];
     __shared__ float wsum[32], csum;
-    __shared__ int fill, base, last;
+    __shared__ int last;
     if (P.counters[kCTwoPass] == 0) return;
     const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + tid; k < (int64_t)P.counters[kCBlocks]; k += gridDim.x * blockDim.x)
+        P.hb_arrive[k] = 0;  // for the second pass
     FrameDev &f = P.frames[P.active[blockIdx.x / CL]];
     const bool act = f.status == kRansac && f.step_samples > 0 && f.m_blocks > 0;  // uniform over the cluster
     if (act) {
@@ -1478,38 +1500,31 @@ __global__ void __launch_bounds__(1024) k_prune(Pools P) {
             for (int r = lane; r < R; r += 32) cut[r] = r >= from ? c : inf;
         }
         __syncthreads();
-        // Each CTA keeps from its slice of the hypotheses, four a thread at a time.
+        // Each CTA keeps from its slice of the hypotheses; few are left, so a warp that
+        // keeps some takes their places in the list with one atomic.
         const int nh = f.hyp_count;
         const int64_t hb = f.hyp_base;
         const int i1 = (int)((int64_t)nh * (rank + 1) / CL);
-        for (int i0 = (int)((int64_t)nh * rank / CL); i0 < i1; i0 += 4 * blockDim.x) {
-            unsigned keep = 0;
+        for (int i0 = (int)((int64_t)nh * rank / CL) + 32 * w; i0 < i1; i0 += 4 * (int)blockDim.x) {
+            bool keep[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int i = i0 + u * (int)blockDim.x + tid;
-                if (i < i1 && (P.hS32[hb + i] < cut[R == 1 ? 0 : round_of(f, P.hId[hb + i])] || (unsigned)i == leader))
-                    keep |= 1u << u;
+                const int i = i0 + u * (int)blockDim.x + lane;
+                keep[u] = i < i1 && (P.hS32[hb + i] < cut[R == 1 ? 0 : round_of(f, P.hId[hb + i])] || (unsigned)i == leader);
             }
-            if (tid == 0) fill = 0;
-            __syncthreads();
-            const int mine = __popc(keep);
-            int at = mine;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, at, o);
-                if (lane >= o) at += u;
+            for (int u = 0; u < 4; ++u) {
+                const unsigned b = __ballot_sync(0xffffffffu, keep[u]);
+                if (!b) continue;
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&f.surv, __popc(b));
+                at = __shfl_sync(0xffffffffu, at, 0) + __popc(b & ((1u << lane) - 1u));
+                if (keep[u]) P.surv[hb + at] = i0 + u * (int)blockDim.x + lane;
             }
-            int w0 = 0;
-            if (lane == 31 && at) w0 = atomicAdd(&fill, at);
-            w0 = __shfl_sync(0xffffffffu, w0, 31);
-            __syncthreads();
-            if (tid == 0) base = fill ? atomicAdd(&f.surv, fill) : 0;
-            __syncthreads();
-            at += w0 - mine + base;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (keep >> u & 1u) P.surv[hb + at++] = i0 + u * (int)blockDim.x + tid;
         }
+        // The leader, where one was needed, has been read by every CTA.
+        if (rank == 0)
+            for (int r = tid; r < R; r += blockDim.x) f.round_min[r] = ~0ull;
     }
     // The launch's last CTA plans the second pass.
     __threadfence();
@@ -1558,7 +1573,45 @@ __device__ __forceinline__ unsigned long long cand_key(float s, float t, float i
 
 __device__ __forceinline__ float cand_limit(float t) { return t + (t * (1.0f / 16384.0f) + 1.0f); }
 
-__global__ void k_select(Pools P) {
+// Work items of the re-rank: (frame, group of candidates, point chunk).
+__device__ __forceinline__ void rescore_plan(const Pools &P) {
+    __shared__ int64_t sh[33];
+    const int a = threadIdx.x;
+    if (P.n_active <= 32 && a >= 32) return;  // one warp's work, without block barriers
+    int64_t items = 0;
+    if (a < P.n_active) {
+        const int slot = P.active[a];
+        FrameDev &f = P.frames[slot];
+        if (f.status == kRansac && f.step_samples > 0) {
+            const int64_t want = (f.n + 2047) / 2048;
+            const int nrc = (int)(want < kMaxRChunks ? want : kMaxRChunks);
+            f.n_rchunks = nrc;
+            f.rchunk = (f.n + nrc - 1) / nrc;
+            items = (int64_t)((f.cand_count + kRescoreGroup - 1) / kRescoreGroup) * nrc;
+        }
+    }
+    int64_t tot, ex;
+    if (P.n_active <= 32) {
+        int64_t incl = items;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (a >= o) incl += u;
+        }
+        tot = __shfl_sync(0xffffffffu, incl, 31);
+        ex = incl - items;
+    } else {
+        ex = block_exclusive_scan(items, sh, tot);
+    }
+    if (a < P.n_active) P.ritem_prefix[a] = ex;
+    if (a == 0) {
+        P.ritem_prefix[P.n_active] = tot;
+        P.counters[kCRescoreTotal] = (unsigned long long)tot;
+    }
+}
+
+// One CTA per frame; the launch's last CTA to finish plans the re-rank.
+__device__ __forceinline__ void select_frame(const Pools &P) {
     __shared__ float thr[kMaxRoundsPerStep], inv_safe[kMaxRoundsPerStep];
     __shared__ unsigned hist[256];
     __shared__ int cnt0, fill, mode, drop_safe;
@@ -1569,15 +1622,32 @@ __global__ void k_select(Pools P) {
     FrameDev &f = P.frames[slot];
     if (f.status != kRansac || f.step_samples == 0) return;
     const int R = (int)f.step_rounds;
-    if (threadIdx.x == 0) {
-        float pm = f.found ? (float)(f.best_score / f.sq_thr) : __int_as_float(0x7f800000);
-        for (int r = 0; r < R; ++r) {
-            const unsigned long long k = f.round_min[r];
-            const float rm = k == ~0ull ? __int_as_float(0x7f800000) : __uint_as_float((unsigned)(k >> 32));
-            pm = fminf(pm, rm);
-            thr[r] = pm;
-            inv_safe[r] = __frcp_rn(pm * (1.0f / 32768.0f) + 0.5f);
+    if (threadIdx.x < 32) {  // running minimum over the rounds, four a lane
+        const float inf = __int_as_float(0x7f800000);
+        float m[4], pm = inf;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int r = 4 * (int)threadIdx.x + u;
+            const unsigned long long k = r < R ? f.round_min[r] : ~0ull;
+            pm = fminf(pm, k == ~0ull ? inf : __uint_as_float((unsigned)(k >> 32)));
+            m[u] = pm;
         }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_up_sync(0xffffffffu, pm, o);
+            if ((int)threadIdx.x >= o) pm = fminf(pm, v);
+        }
+        float before = __shfl_up_sync(0xffffffffu, pm, 1);
+        if (threadIdx.x == 0) before = inf;
+        if (f.found) before = fminf(before, (float)(f.best_score / f.sq_thr));
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float t = fminf(before, m[u]);
+            thr[4 * threadIdx.x + u] = t;
+            inv_safe[4 * threadIdx.x + u] = __frcp_rn(t * (1.0f / 32768.0f) + 0.5f);
+        }
+    }
+    if (threadIdx.x == 0) {
         cnt0 = 0;
         fill = 0;
         drop_safe = 0;
@@ -1694,37 +1764,24 @@ __global__ void k_select(Pools P) {
             }
         }
         const int c = atomicAdd(&fill, 1);
-        if (c < cap) P.cHyp[base + c] = i;
+        if (c < cap) {
+            P.cHyp[base + c] = i;
+            P.c_arrive[base + c] = 0;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0 && drop_safe) f.overflow = 1;
 }
-
-__global__ void k_rescore_plan(Pools P) {
-    __shared__ int64_t sh[33];
-    const int a = threadIdx.x;
-    int64_t items = 0;
-    if (a < P.n_active) {
-        const int slot = P.active[a];
-        FrameDev &f = P.frames[slot];
-        if (f.status == kRansac && f.step_samples > 0) {
-            const int64_t want = (f.n + 2047) / 2048;
-            const int nrc = (int)(want < kMaxRChunks ? want : kMaxRChunks);
-            f.n_rchunks = nrc;
-            f.rchunk = (f.n + nrc - 1) / nrc;
-            items = (int64_t)((f.cand_count + kRescoreGroup - 1) / kRescoreGroup) * nrc;
-        }
-    }
-    // The step's candidates lie in [0, claimed) of the pool: arrival counters zeroed by the block.
-    const int64_t claimed = min((int64_t)P.counters[kCCandNext], P.cand_cap);
-    for (int64_t c = threadIdx.x; c < claimed; c += blockDim.x) P.c_arrive[c] = 0;
-    int64_t tot;
-    const int64_t ex = block_exclusive_scan(items, sh, tot);
-    if (a < P.n_active) P.ritem_prefix[a] = ex;
-    if (a == 0) {
-        P.ritem_prefix[P.n_active] = tot;
-        P.counters[kCRescoreTotal] = (unsigned long long)tot;
-    }
+__global__ void __launch_bounds__(1024) k_select(Pools P) {
+    __shared__ int last;
+    select_frame(P);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&P.counters[kCSelected], 1ull) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    rescore_plan(P);
 }
 
 // Exact FP64 truncated MSAC of a group of up to kRescoreGroup candidates of a
@@ -1837,7 +1894,7 @@ __global__ void __launch_bounds__(256) k_rescore(Pools P) {
 // solution) replaces the running best only if strictly better; after each
 // round the stop rule uses the running best's inlier count. One CTA per frame:
 // the per-round minima are found in parallel, the round walk is sequential.
-__global__ void __launch_bounds__(256) k_finalize(Pools P) {
+__device__ __forceinline__ void finalize_frame(const Pools &P) {
     __shared__ unsigned long long rmin[kMaxRoundsPerStep];   // ordered FP64 score
     __shared__ unsigned long long rid[kMaxRoundsPerStep];    // hypothesis id
     __shared__ int rwin[kMaxRoundsPerStep];                  // candidate index
@@ -1889,27 +1946,33 @@ __global__ void __launch_bounds__(256) k_finalize(Pools P) {
     bool stop = false;
     if (threadIdx.x == 0) {
         f.rescored += C;
-        int64_t r_end = f.step_rounds;
-        for (int64_t r = 0; r < f.step_rounds; ++r) {
+        // The samples needed change only with the best model.
+        const int64_t B = f.B, first = f.step_first, least = f.min_samples, cap = f.max_total, R = f.step_rounds;
+        int found = f.found;
+        double best = f.best_score;
+        int64_t r_end = R;
+        int64_t need = forced ? 0 : needed_samples(found ? f.best_count : 0, f.n, f.log_missing, f.trials_mult, f.quirk);
+        for (int64_t r = 0; r < R; ++r) {
             const int c = rwin[r];
             if (c >= 0) {
                 const int64_t cs = f.cand_base + c;
                 const double bs = P.cS64[cs];
-                if (!f.found || bs < f.best_score) {
+                if (!found || bs < best) {
                     const int64_t bid = (int64_t)rid[r];
-                    f.found = 1;
-                    f.best_score = bs;
-                    f.best_count = P.cCnt[cs];
+                    const int64_t count = P.cCnt[cs];
+                    found = f.found = 1;
+                    best = f.best_score = bs;
+                    f.best_count = count;
                     f.best_sample = bid >> 2;
                     f.best_sol = (int32_t)(bid & 3);
                     const double *Pp = P.hP64 + 12 * (f.hyp_base + P.cHyp[cs]);
                     for (int e = 0; e < 12; ++e) f.best_P[e] = Pp[e];
+                    if (!forced) need = needed_samples(count, f.n, f.log_missing, f.trials_mult, f.quirk);
                 }
             }
             if (forced) continue;
-            const int64_t after = f.step_first + (r + 1) * f.B;
-            const int64_t need = needed_samples(f.found ? f.best_count : 0, f.n, f.log_missing, f.trials_mult, f.quirk);
-            if ((after > need && after >= f.min_samples) || after >= f.max_total) {
+            const int64_t after = first + (r + 1) * B;
+            if ((after > need && after >= least) || after >= cap) {
                 stop = true;
                 r_end = r + 1;
                 break;
@@ -1924,7 +1987,10 @@ __global__ void __launch_bounds__(256) k_finalize(Pools P) {
     if (r_end < f.step_rounds) {
         const int64_t end_id = 4 * (f.step_first + r_end * f.B);
         int mine = 0;
-        for (int i = threadIdx.x; i < f.hyp_count; i += blockDim.x) mine += P.hId[f.hyp_base + i] < end_id ? 1 : 0;
+        const int nh = f.hyp_count;
+        const int64_t *id = P.hId + f.hyp_base;
+#pragma unroll 8
+        for (int i = threadIdx.x; i < nh; i += blockDim.x) mine += id[i] < end_id ? 1 : 0;
         mine = warp_sum(mine);
         if ((threadIdx.x & 31) == 0) atomicAdd(&hyps, mine);
     }
@@ -1950,6 +2016,30 @@ __global__ void __launch_bounds__(256) k_finalize(Pools P) {
     } else {
         atomicAdd(&P.counters[kCStillRansac], 1ull);
     }
+}
+__global__ void __launch_bounds__(256) k_finalize(Pools P) { finalize_frame(P); }
+
+// The same at the end of a captured loop's body: the launch's last CTA to finish
+// closes the step and decides whether the loop goes on -- while any frame is still in
+// RANSAC, with a step limit that turns a runaway loop into an error.
+__global__ void __launch_bounds__(256) k_finalize_loop(Pools P, cudaGraphConditionalHandle h,
+                                                       unsigned long long max_steps) {
+    finalize_frame(P);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&P.counters[kCFinal], 1ull) != gridDim.x - 1) return;
+    __threadfence();
+    volatile unsigned long long *C = P.counters;
+    const unsigned long long steps = C[kCSteps] + 1;
+    C[kCSteps] = steps;
+    unsigned v = C[kCStillRansac] > 0 ? 1u : 0u;
+    if (v && steps >= max_steps) {
+        flag_error(P, kErrOverflow);
+        v = 0u;
+    }
+    if (C[kCError] & kErrTimeout) v = 0u;
+    cudaGraphSetConditional(h, v);
 }
 
 // ------------------------------------------------------------- inliers -----
@@ -2504,20 +2594,6 @@ __global__ void k_debug_bounded_wait(unsigned long long *counters, uint32_t poll
 __global__ void k_gather_status(Pools P, int32_t *out) {
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < P.n_active; a += gridDim.x * blockDim.x)
         out[a] = P.frames[P.active[a]].status;
-}
-
-// ----------------------------------------------------------- loop control --
-// Body tail of the captured batch loop: continue while any frame is still in
-// RANSAC, with a step limit that turns a runaway loop into an error.
-__global__ void k_loop_ctl(Pools P, cudaGraphConditionalHandle h, unsigned long long max_steps) {
-    const unsigned long long steps = ++P.counters[kCSteps];
-    unsigned v = P.counters[kCStillRansac] > 0 ? 1u : 0u;
-    if (v && steps >= max_steps) {
-        flag_error(P, kErrOverflow);
-        v = 0u;
-    }
-    if (P.counters[kCError] & kErrTimeout) v = 0u;
-    cudaGraphSetConditional(h, v);
 }
 
 // Frames of Q waiting for their data start RANSAC (their points are in the
