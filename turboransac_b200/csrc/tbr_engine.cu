@@ -215,6 +215,9 @@ class Engine {
     cudaEvent_t ev_lm_fork = nullptr, ev_lm_join = nullptr;
     void *d_stage_alias = nullptr;              // device address of the pinned staging buffer
     cudaEvent_t ev_done = nullptr;              // a submitted batch's downloads have landed
+    uint8_t *h_masks = nullptr;                 // pinned: inlier masks of a synchronous call (k_publish)
+    size_t h_masks_bytes = 0;
+    int64_t *h_mask_at = nullptr;               // pinned: each frame's place in h_masks
     cudaStream_t stream_out = nullptr;          // inlier masks of a collected batch
     // Ingestion of the first part of a host batch runs on stream_in, beside
     // whatever the context stream still runs (it writes only the new frames'
@@ -266,6 +269,8 @@ class Engine {
         if (h_stage) cudaFreeHost(h_stage);
         if (h_counters) cudaFreeHost(h_counters);
         if (h_results) cudaFreeHost(h_results);
+        if (h_masks) cudaFreeHost(h_masks);
+        if (h_mask_at) cudaFreeHost(h_mask_at);
         if (d_replay) cudaFree(d_replay);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
@@ -383,6 +388,7 @@ class Engine {
         TBR_CUDA(cudaMemsetAsync(P.frames, 0, sizeof(FrameDev) * max_frames, stream));
         TBR_CUDA(cudaMallocHost(&h_counters, 8 * kCNum));
         TBR_CUDA(cudaMallocHost(&h_results, sizeof(FrameResult) * kMaxActive));
+        TBR_CUDA(cudaMallocHost(&h_mask_at, sizeof(int64_t) * kMaxActive));
         TBR_CUDA(cudaMallocHost(&spare.h_counters, 8 * kCNum));
         TBR_CUDA(cudaMallocHost(&spare.h_results, sizeof(FrameResult) * kMaxActive));
         blocks.reset(max_blocks);
@@ -417,6 +423,17 @@ class Engine {
             cudaGetLastError();
             d_stage_alias = nullptr;
         }
+        return TBR_OK;
+    }
+
+    tbr_status ensure_masks(size_t bytes) {
+        if (bytes <= h_masks_bytes) return TBR_OK;
+        if (h_masks) cudaFreeHost(h_masks);
+        h_masks = nullptr;
+        const size_t nb = std::max(bytes, 2 * h_masks_bytes);
+        h_masks_bytes = 0;
+        TBR_CUDA(cudaMallocHost(&h_masks, nb));
+        h_masks_bytes = nb;
         return TBR_OK;
     }
 
@@ -932,116 +949,6 @@ static tbr_status upload_staged(Engine &E, const StagedAdmission &A) {
     return upload_records(E, A);
 }
 
-// Host copies and uploads in groups of consecutive frames of a run, so that
-// the link moves one group while the host threads copy the next: copy threads
-// take 1 MiB pieces in group order, and this thread issues a group's upload as
-// soon as its last piece is in.
-// Large frames whose arrays are already page-locked go up directly, without a
-// host copy (below ~512 KiB a copy into staging and a shared upload cost less
-// than an upload call of their own).
-constexpr size_t kDirectUploadBytes = 512u << 10;
-static bool page_locked(const void *p) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return at.type == cudaMemoryTypeHost;
-}
-static bool direct_upload(const StagedAdmission &A, size_t i) {
-    return A.jobs[2 * i].bytes + A.jobs[2 * i + 1].bytes >= kDirectUploadBytes && page_locked(A.jobs[2 * i].src) &&
-           page_locked(A.jobs[2 * i + 1].src);
-}
-
-static tbr_status copy_and_upload_overlapped(Engine &E, const StagedAdmission &A) {
-    constexpr size_t kGroupBytes = 8u << 20, kPiece = 1u << 20;
-    struct Group {
-        size_t run, i, j;  // frames i .. j-1 of run
-    };
-    std::vector<char> direct(A.devs.size(), 0);
-    for (size_t i = 0; i < A.devs.size(); ++i) {
-        direct[i] = direct_upload(A, i);
-        if (direct[i]) {
-            const size_t q0 = (size_t)A.devs[i].blk_off * kSub;
-            TBR_CUDA(cudaMemcpyAsync((void *)(E.P.uv64 + 2 * q0), A.jobs[2 * i].src, A.jobs[2 * i].bytes,
-                                     cudaMemcpyHostToDevice, E.stream));
-            TBR_CUDA(cudaMemcpyAsync((void *)(E.P.X64 + 3 * q0), A.jobs[2 * i + 1].src, A.jobs[2 * i + 1].bytes,
-                                     cudaMemcpyHostToDevice, E.stream));
-        }
-    }
-    std::vector<Group> groups;
-    size_t total = 0;
-    for (size_t r = 0; r < A.runs.size(); ++r)
-        for (size_t i = A.span[r].first; i <= A.span[r].second;) {
-            if (direct[i]) {
-                ++i;
-                continue;
-            }
-            size_t j = i, bytes = 0;
-            while (j <= A.span[r].second && !direct[j] && (j == i || bytes < kGroupBytes)) {
-                bytes += A.jobs[2 * j].bytes + A.jobs[2 * j + 1].bytes;
-                ++j;
-            }
-            groups.push_back({r, i, j});
-            total += bytes;
-            i = j;
-        }
-    auto upload = [&](const Group &g) -> tbr_status {
-        const auto &run = A.runs[g.run];
-        // points [p0, p1) of the run: the group's frames with their padding
-        const size_t p0 = (size_t)(A.devs[g.i].blk_off - run.b0) * kSub;
-        const size_t p1 = (size_t)(A.devs[g.j - 1].blk_off + A.devs[g.j - 1].n_blocks - run.b0) * kSub;
-        const size_t q0 = (size_t)run.b0 * kSub + p0;
-        TBR_CUDA(cudaMemcpyAsync((void *)(E.P.uv64 + 2 * q0), run.huv + 16 * p0, 16 * (p1 - p0),
-                                 cudaMemcpyHostToDevice, E.stream));
-        TBR_CUDA(cudaMemcpyAsync((void *)(E.P.X64 + 3 * q0), run.hxyz + 24 * p0, 24 * (p1 - p0),
-                                 cudaMemcpyHostToDevice, E.stream));
-        return TBR_OK;
-    };
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const int T = (int)std::min<size_t>(std::min(8u, hw), total / (4 * kPiece));
-    if (T <= 1) {
-        for (auto &g : groups) {
-            for (size_t k = 2 * g.i; k < 2 * g.j; ++k) std::memcpy(A.jobs[k].dst, A.jobs[k].src, A.jobs[k].bytes);
-            tbr_status st = upload(g);
-            if (st) return st;
-        }
-        return upload_records(E, A);
-    }
-    struct Piece {
-        CopyJob job;
-        size_t group;
-    };
-    std::vector<Piece> pieces;
-    std::unique_ptr<std::atomic<int>[]> left(new std::atomic<int>[groups.size()]);
-    for (size_t g = 0; g < groups.size(); ++g) {
-        int cnt = 0;
-        for (size_t k = 2 * groups[g].i; k < 2 * groups[g].j; ++k)
-            for (size_t o = 0; o < A.jobs[k].bytes; o += kPiece, ++cnt)
-                pieces.push_back({{(char *)A.jobs[k].dst + o, (const char *)A.jobs[k].src + o,
-                                   std::min(kPiece, A.jobs[k].bytes - o)},
-                                  g});
-        left[g].store(cnt, std::memory_order_relaxed);
-    }
-    std::atomic<size_t> next{0};
-    auto work = [&]() {
-        for (size_t k; (k = next.fetch_add(1)) < pieces.size();) {
-            std::memcpy(pieces[k].job.dst, pieces[k].job.src, pieces[k].job.bytes);
-            left[pieces[k].group].fetch_sub(1, std::memory_order_release);
-        }
-    };
-    std::vector<std::thread> th;
-    for (int t = 0; t < T; ++t) th.emplace_back(work);
-    tbr_status st = TBR_OK;
-    for (size_t g = 0; g < groups.size(); ++g) {
-        while (left[g].load(std::memory_order_acquire) > 0) std::this_thread::yield();
-        if (st == TBR_OK) st = upload(groups[g]);
-    }
-    for (auto &x : th) x.join();
-    if (st) return st;
-    return upload_records(E, A);
-}
-
 // ------------------------------------------------------ ingestion tables --
 // Tiles of one (source, pool destination) row, at most `tile` bytes each.
 static void add_row_tiles(std::vector<IngestTile> &v, const void *src, const void *dst, size_t bytes, size_t tile) {
@@ -1259,47 +1166,103 @@ static tbr_status admit_host_frames(Engine &E, const std::vector<FrameHost> &fr,
     return st;
 }
 
+// Small host admissions (one frame, or frames below kZeroCopyMinBytes together): one
+// kernel reads records and points from page-locked memory -- the staging buffer, or
+// the caller's own arrays where they are page-locked and large enough for the
+// query to cost less than the copy -- and does the whole preparation
+// (k_admit_points); with `clear` it also zeroes the counters.
+constexpr size_t kMappedQueryBytes = 128u << 10;
+
+// Copies a frame's arrays into its staging place, or finds the caller's page-locked
+// ones; src: their two addresses as the device sees them.
+static void stage_or_map(Engine &E, const StagedAdmission &A, size_t i, std::vector<CopyJob> &copies, const void **src) {
+    const CopyJob &u = A.jobs[2 * i], &x = A.jobs[2 * i + 1];
+    const void *mu = nullptr, *mx = nullptr;
+    if (u.bytes + x.bytes >= kMappedQueryBytes && (mu = mapped_address(u.src))) mx = mapped_address(x.src);
+    if (mu && mx) {
+        src[0] = mu;
+        src[1] = mx;
+        return;
+    }
+    copies.push_back(u);
+    copies.push_back(x);
+    src[0] = (const char *)E.d_stage_alias + ((const char *)u.dst - (const char *)E.h_stage);
+    src[1] = (const char *)E.d_stage_alias + ((const char *)x.dst - (const char *)E.h_stage);
+}
+template <class T>
+static T *stage_alias(Engine &E, T *p) {  // the staging buffer's address as the device sees it
+    return (T *)((char *)E.d_stage_alias + ((char *)p - (char *)E.h_stage));
+}
+
+static tbr_status admit_small(Engine &E, const std::vector<FrameHost> &fr, const RunOptions &o, std::vector<int> &slots,
+                              int64_t &max_n, std::vector<FrameDev> *host_devs, bool clear) {
+    const size_t n = fr.size(), tab = stage_bytes(fr);
+    tbr_status st = E.ensure_stage(tab + 16 * n);
+    if (st) return st;
+    if (!E.d_stage_alias) return fail(TBR_ERR_CUDA, "staging buffer has no device address");
+    StagedAdmission A;
+    st = stage_frames(E, fr, o, (char *)E.h_stage, A, false, true);
+    if (st) return st;
+    // The caller releases these, whatever happens next.
+    slots = A.slots;
+    max_n = A.max_n;
+    if (host_devs) *host_devs = A.devs;
+    const void **src = (const void **)((char *)E.h_stage + tab);
+    std::vector<CopyJob> copies;
+    for (size_t i = 0; i < n; ++i) stage_or_map(E, A, i, copies, src + 2 * i);
+    parallel_copy(copies);
+    k_admit_points<<<(int)n * kAdmitCtas, kAdmitThreads, 0, E.stream>>>(
+        E.P, stage_alias(E, A.hd), stage_alias(E, A.ha), (const char *const *)stage_alias(E, src), E.d_active,
+        clear ? 1 : 0);
+    TBR_CUDA(cudaGetLastError());
+    E.P.n_active = (int32_t)n;
+    return TBR_OK;
+}
+
 // Both halves through the context's own staging buffer. With device_points the
 // frames' point arrays are device memory of this GPU: they are copied into the
 // pool by one kernel, with no host staging. Multi-frame host batches of some
-// size are ingested zero-copy (admit_host_frames); a small admission uploads
-// its staging runs with copy calls.
+// size are ingested zero-copy (admit_host_frames), smaller ones and single frames by
+// admit_small, which also prepares them (*prepared).
 static tbr_status admit_frames(Engine &E, const std::vector<FrameHost> &fr, const RunOptions &o,
-                               std::vector<int> &slots, int64_t &max_n, std::vector<FrameDev> *host_devs = nullptr,
-                               bool device_points = false) {
+                               std::vector<int> &slots, int64_t &max_n, bool *prepared,
+                               std::vector<FrameDev> *host_devs = nullptr, bool device_points = false,
+                               bool clear = false) {
+    *prepared = false;
     size_t in_bytes = 0;
     for (auto &f : fr) in_bytes += 40 * (size_t)f.n;
+    const bool small = !device_points && (fr.size() < 2 || in_bytes < kZeroCopyMinBytes);
+    if (clear && !small) TBR_CUDA(cudaMemsetAsync(E.P.counters, 0, 8 * kCNum, E.stream));
     if (!device_points && fr.size() >= 2 && in_bytes >= kZeroCopyMinBytes) {
         std::vector<FrameDev> d;
         tbr_status st = admit_host_frames(E, fr, o, slots, max_n, d, false);
         if (host_devs) *host_devs = d;
         return st;
     }
+    if (!device_points) {
+        *prepared = true;
+        return admit_small(E, fr, o, slots, max_n, host_devs, clear);
+    }
     auto r256 = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t rec = r256(sizeof(FrameDev) * fr.size()) + r256(4 * fr.size());
-    tbr_status st = E.ensure_stage(device_points ? rec + Engine::kIngestTableBytes : stage_bytes(fr));
+    tbr_status st = E.ensure_stage(rec + Engine::kIngestTableBytes);
     if (st) return st;
     StagedAdmission A;
-    st = stage_frames(E, fr, o, (char *)E.h_stage, A, false, !device_points);
+    st = stage_frames(E, fr, o, (char *)E.h_stage, A, false, false);
     if (st) return st;
     // The caller releases these, whatever happens next.
     slots = A.slots;
     max_n = A.max_n;
     if (host_devs) *host_devs = A.devs;
-    if (device_points) {
-        std::vector<IngestTile> t;
-        const size_t tile = ingest_tile_bytes(fr);
-        for (size_t i = 0; i < fr.size(); ++i) add_frame_tiles(t, E, A.devs[i], fr[i].n, fr[i].uv, fr[i].xyz, tile);
-        size_t off = 0;
-        const int64_t *d = put_table(E, (char *)E.h_stage + rec, off, t, E.d_ingest, E.stream);
-        if (!d) return fail(TBR_ERR_CUDA, "ingestion table upload failed");
-        k_ingest<<<E.num_sms * 2, 256, 0, E.stream>>>(d);
-        TBR_CUDA(cudaGetLastError());
-        st = upload_records(E, A);
-    } else {
-        st = copy_and_upload_overlapped(E, A);
-    }
-    return st;
+    std::vector<IngestTile> t;
+    const size_t tile = ingest_tile_bytes(fr);
+    for (size_t i = 0; i < fr.size(); ++i) add_frame_tiles(t, E, A.devs[i], fr[i].n, fr[i].uv, fr[i].xyz, tile);
+    size_t off = 0;
+    const int64_t *d = put_table(E, (char *)E.h_stage + rec, off, t, E.d_ingest, E.stream);
+    if (!d) return fail(TBR_ERR_CUDA, "ingestion table upload failed");
+    k_ingest<<<E.num_sms * 2, 256, 0, E.stream>>>(d);
+    TBR_CUDA(cudaGetLastError());
+    return upload_records(E, A);
 }
 
 // Results of `slots` into `out` (host), through one packed download.
@@ -1489,10 +1452,9 @@ void tbr_context_destroy(tbr_context *ctx) {
 // next (the caller releases them).
 static tbr_status enqueue_frames(Engine &E, const std::vector<FrameHost> &fr, const RunOptions &o,
                                  std::vector<int> &slots, std::vector<FrameDev> &devs, bool device_points,
-                                 bool behind = false) {
+                                 bool behind = false, const std::vector<uint8_t *> *masks = nullptr) {
     int64_t max_n = 0;
     TBR_CUDA(cudaSetDevice(E.device));
-    TBR_CUDA(cudaMemsetAsync(E.P.counters, 0, 8 * kCNum, E.stream));
     size_t in_bytes = 0;
     double pairs = 0.0;
     for (auto &f : fr) {
@@ -1502,27 +1464,38 @@ static tbr_status enqueue_frames(Engine &E, const std::vector<FrameHost> &fr, co
     E.P.prune = want_prune(pairs);
     tbr_status st;
     if (!device_points && fr.size() >= 2 && in_bytes >= kStaggerMinBytes) {
+        TBR_CUDA(cudaMemsetAsync(E.P.counters, 0, 8 * kCNum, E.stream));
         st = admit_host_frames(E, fr, o, slots, max_n, devs, true, !behind);
     } else {
-        st = admit_frames(E, fr, o, slots, max_n, &devs, device_points);
+        bool prepared = false;
+        st = admit_frames(E, fr, o, slots, max_n, &prepared, &devs, device_points, true);
         if (st == TBR_OK) {
             TBR_CUDA(cudaEventRecord(E.ev0, E.stream));
-            E.launch_prep((int)slots.size(), max_n);
+            if (!prepared) E.launch_prep((int)slots.size(), max_n);
             E.pp = o.pp;
             st = E.launch_graph((int)slots.size(), o.hr);
         }
     }
     if (st) return st;
     TBR_CUDA(cudaEventRecord(E.ev1, E.stream));
-    // Everything the caller gets back in one round trip: the results in the
-    // order of the active list (= slots) and the counters.
+    // Everything the caller gets back, written to page-locked memory by one
+    // kernel: the results in the order of the active list (= slots), the
+    // counters, and the masks that are wanted.
     const int n = (int)slots.size();
-    k_gather_results<<<(int)std::min<size_t>(1024, (n * (sizeof(FrameResult) / 8) + 255) / 256), 256, 0,
-                       E.stream>>>(E.P.results, E.d_active, n, E.d_res_stage);
+    bool any = false;
+    if (masks) {
+        size_t at = 0;
+        for (int i = 0; i < n; ++i) {
+            const bool want = (size_t)i < masks->size() && (*masks)[i];
+            E.h_mask_at[i] = want ? (int64_t)at : -1;
+            if (want) at += ((size_t)fr[i].n + 15) & ~size_t(15);
+            any = any || want;
+        }
+        if (any && (st = E.ensure_masks(at))) return st;
+    }
+    k_publish<<<dim3(n, any ? (n == 1 ? 8 : 2) : 1), 256, 0, E.stream>>>(E.P, E.d_active, E.h_results, E.h_counters,
+                                                                       E.h_masks, any ? E.h_mask_at : nullptr);
     TBR_CUDA(cudaGetLastError());
-    TBR_CUDA(cudaMemcpyAsync(E.h_results, E.d_res_stage, sizeof(FrameResult) * n, cudaMemcpyDeviceToHost,
-                             E.stream));
-    TBR_CUDA(cudaMemcpyAsync(E.h_counters, E.P.counters, 8 * kCNum, cudaMemcpyDeviceToHost, E.stream));
     return TBR_OK;
 }
 
@@ -1532,15 +1505,13 @@ static tbr_status estimate_frames(tbr_context *ctx, const std::vector<FrameHost>
     Engine &E = ctx->E;
     std::vector<int> slots;
     std::vector<FrameDev> devs;
-    tbr_status st = enqueue_frames(E, fr, o, slots, devs, device_points);
+    tbr_status st = enqueue_frames(E, fr, o, slots, devs, device_points, false, &masks);
     if (st == TBR_OK) {
-        for (size_t i = 0; i < slots.size(); ++i)
-            if (i < masks.size() && masks[i])
-                TBR_CUDA(cudaMemcpyAsync(masks[i], E.P.mask + devs[i].blk_off * kSub, fr[i].n,
-                                         cudaMemcpyDeviceToHost, E.stream));
         TBR_CUDA(cudaStreamSynchronize(E.stream));
         st = run_status(E.h_counters);
         if (st == TBR_OK) {
+            for (size_t i = 0; i < slots.size(); ++i)
+                if (i < masks.size() && masks[i]) std::memcpy(masks[i], E.h_masks + E.h_mask_at[i], fr[i].n);
             res.assign(E.h_results, E.h_results + slots.size());
             if (steps_out) *steps_out = (int)E.h_counters[kCSteps];
             float ms = 0.f;
@@ -1878,36 +1849,37 @@ tbr_status tbr_get_inliers(tbr_context *ctx, const double q[4], const double t[3
     const int64_t nb = (n + kSub - 1) / kSub;
     const int64_t off = E.blocks.alloc(nb);
     if (off < 0) return fail(TBR_ERR_OOM, "point workspace exhausted");
-    const int64_t p0 = off * kSub;
-    tbr_status st = E.ensure_stage(40 * n + 1024 + n);
-    if (st) { E.blocks.release(off, nb); return st; }
+    E.blocks.release(off, nb);  // (a request larger than the workspace is refused; the points stay in host memory)
+    // [x | X | pose | mask | counts] in page-locked memory, read and written by the kernel.
+    const int grid = (int)std::min<int64_t>(E.num_sms * 4, (n + kMaskPts - 1) / kMaskPts);
+    const size_t room = (size_t)((n + kMaskPts - 1) / kMaskPts) * kMaskPts;
+    tbr_status st = E.ensure_stage(40 * (size_t)n + 64 + room + 4 * (size_t)grid + 256);
+    if (st) return st;
+    if (!E.d_stage_alias) return fail(TBR_ERR_CUDA, "staging buffer has no device address");
     char *h = (char *)E.h_stage;
-    std::memcpy(h, x, 16 * n);
-    std::memcpy(h + 16 * n, X, 24 * n);
-    double *hq = (double *)(h + 40 * n);
+    const double *dx = nullptr, *dX = nullptr;
+    if (40 * (size_t)n >= kMappedQueryBytes && (dx = (const double *)mapped_address(x)))
+        dX = (const double *)mapped_address(X);
+    if (!dx || !dX) {
+        // x first, rounded up to 16 bytes (16 n always is)
+        parallel_copy({{h, x, 16 * (size_t)n}, {h + 16 * n, X, 24 * (size_t)n}});
+        dx = (const double *)stage_alias(E, h);
+        dX = (const double *)stage_alias(E, h + 16 * n);
+    }
+    double *hq = (double *)(h + (((size_t)40 * n + 63) & ~size_t(63)));
     for (int k = 0; k < 4; ++k) hq[k] = q[k];
     for (int k = 0; k < 3; ++k) hq[4 + k] = t[k];
-    // x goes to the normalized-coordinate pool, X to the world-point pool; the
-    // pose rides in the first hypothesis slot.
-    TBR_CUDA(cudaMemcpyAsync(E.P.xn64 + 2 * p0, h, 16 * n, cudaMemcpyHostToDevice, E.stream));
-    TBR_CUDA(cudaMemcpyAsync((void *)(E.P.X64 + 3 * p0), h + 16 * n, 24 * n, cudaMemcpyHostToDevice, E.stream));
-    TBR_CUDA(cudaMemcpyAsync(E.P.hP64, hq, 7 * 8, cudaMemcpyHostToDevice, E.stream));
-    TBR_CUDA(cudaMemsetAsync(E.P.counters + kCWorkPairs, 0, 8, E.stream));
-    const int grid = (int)std::min<int64_t>(E.num_sms * 4, (n + 255) / 256);
-    k_pose_mask<<<grid, 256, 0, E.stream>>>(E.P.xn64 + 2 * p0, E.P.X64 + 3 * p0, n, E.P.hP64, sq_threshold,
-                                            E.P.mask + p0, E.P.counters + kCWorkPairs);
-    st = TBR_OK;
-    if (cudaGetLastError() != cudaSuccess) st = fail(TBR_ERR_CUDA, "k_pose_mask launch failed");
-    uint8_t *hm = (uint8_t *)(h + 40 * n + 64);
-    if (!st) {
-        cudaMemcpyAsync(hm, E.P.mask + p0, n, cudaMemcpyDeviceToHost, E.stream);
-        cudaMemcpyAsync(E.h_counters, E.P.counters, 8 * kCNum, cudaMemcpyDeviceToHost, E.stream);
-    }
-    if (cudaStreamSynchronize(E.stream) != cudaSuccess && !st) st = fail(TBR_ERR_CUDA, "get_inliers failed");
-    E.blocks.release(off, nb);
-    if (st) return st;
+    uint8_t *hm = (uint8_t *)(hq + 8);
+    unsigned *hc = (unsigned *)(hm + room);
+    k_pose_mask<<<grid, kMaskPts, 0, E.stream>>>(dx, dX, n, stage_alias(E, hq), sq_threshold, stage_alias(E, hm),
+                                                 stage_alias(E, hc));
+    TBR_CUDA(cudaGetLastError());
+    TBR_CUDA(cudaStreamSynchronize(E.stream));
     if (inliers) std::memcpy(inliers, hm, n);
-    if (count) *count = (int64_t)E.h_counters[kCWorkPairs];
+    if (count) {
+        *count = 0;
+        for (int k = 0; k < grid; ++k) *count += hc[k];
+    }
     return TBR_OK;
 }
 
@@ -1945,15 +1917,18 @@ tbr_status tbr_bundle_adjust(tbr_context *ctx, const double *x, const double *X,
         if (stats) std::memset(stats, 0, sizeof(*stats));
         return TBR_OK;
     }
-    std::vector<int> slots;
-    int64_t max_n = 0;
-    TBR_CUDA(cudaMemsetAsync(E.P.counters, 0, 8 * kCNum, E.stream));
-    tbr_status st = admit_frames(E, {fh}, o, slots, max_n);
+    // [points | record, slot | start pose | weights] in page-locked memory, read by one kernel.
+    const std::vector<FrameHost> one{fh};
+    const size_t tab = stage_bytes(one), r0_bytes = (sizeof(FrameResult) + 255) & ~size_t(255);
+    tbr_status st = E.ensure_stage(tab + r0_bytes + (weighted ? 8 * (size_t)n : 0) + 64);
     if (st) return st;
-    FrameDev fd;
-    TBR_CUDA(cudaMemcpyAsync(&fd, E.P.frames + slots[0], sizeof(FrameDev), cudaMemcpyDeviceToHost, E.stream));
-    TBR_CUDA(cudaStreamSynchronize(E.stream));
+    if (!E.d_stage_alias) return fail(TBR_ERR_CUDA, "staging buffer has no device address");
+    StagedAdmission A;
+    st = stage_frames(E, one, o, (char *)E.h_stage, A, false, true);
+    if (st) return st;
+    FrameDev &fd = *A.hd;
     fd.status = kLMPending;
+    fd.num_inliers = n;
     fd.lm_force_cluster = 1;
     fd.focal = 1.0;
     for (int k = 0; k < 4; ++k) fd.lm_cam[k] = K[k];
@@ -1961,8 +1936,6 @@ tbr_status tbr_bundle_adjust(tbr_context *ctx, const double *x, const double *X,
     fd.lm_thr = bo.loss_scale;
     fd.lm_loss = loss;
     fd.lm_weighted = weighted ? 1 : 0;
-    if (weighted)
-        TBR_CUDA(cudaMemcpyAsync(E.P.lw64 + fd.blk_off * kSub, weights, 8 * n, cudaMemcpyHostToDevice, E.stream));
     fd.lm_max_iter = (int64_t)bo.max_iterations;
     fd.lm_grad_tol = bo.gradient_tol;
     fd.lm_step_tol = bo.step_tol;
@@ -1970,26 +1943,30 @@ tbr_status tbr_bundle_adjust(tbr_context *ctx, const double *x, const double *X,
     fd.lm_min_lambda = bo.min_lambda;
     fd.lm_max_lambda = bo.max_lambda;
     fd.skip_refine = 0;
-    FrameResult r0;
-    std::memset(&r0, 0, sizeof(r0));
-    for (int k = 0; k < 4; ++k) r0.q[k] = q[k];
-    for (int k = 0; k < 3; ++k) r0.t[k] = t[k];
-    TBR_CUDA(cudaMemcpyAsync(E.P.frames + slots[0], &fd, sizeof(FrameDev), cudaMemcpyHostToDevice, E.stream));
-    TBR_CUDA(cudaMemcpyAsync(E.P.results + slots[0], &r0, sizeof(FrameResult), cudaMemcpyHostToDevice, E.stream));
-    const int bx = (int)std::min<int64_t>(64, std::max<int64_t>(1, (n + 1023) / 1024));
-    k_prep_bounds<<<dim3(bx, 1), 256, 0, E.stream>>>(E.P);
-    k_lm_pack<<<bx, 256, 0, E.stream>>>(E.P);
+    FrameResult *r0 = (FrameResult *)((char *)E.h_stage + tab);
+    std::memset(r0, 0, sizeof(*r0));
+    for (int k = 0; k < 4; ++k) r0->q[k] = q[k];
+    for (int k = 0; k < 3; ++k) r0->t[k] = t[k];
+    std::vector<CopyJob> copies;
+    const void *src[2];
+    stage_or_map(E, A, 0, copies, src);
+    double *hw = (double *)((char *)r0 + r0_bytes);
+    if (weighted) copies.push_back({hw, weights, 8 * (size_t)n});
+    parallel_copy(copies);
+    E.P.n_active = 1;
+    k_admit_lm<<<(int)std::min<int64_t>(32, (n + 511) / 512), 256, 0, E.stream>>>(
+        E.P, stage_alias(E, A.hd), stage_alias(E, r0), A.slots[0], (const char *)src[0], (const char *)src[1],
+        weighted ? (const char *)stage_alias(E, hw) : nullptr, E.d_active);
     cudaEventRecord(E.ev0, E.stream);
     k_lm<<<kLMCluster, kLMThreads, 0, E.stream>>>(E.P);
     cudaEventRecord(E.ev1, E.stream);
+    k_publish<<<1, 256, 0, E.stream>>>(E.P, E.d_active, E.h_results, E.h_counters, nullptr, nullptr);
     st = TBR_OK;
     if (cudaGetLastError() != cudaSuccess) st = fail(TBR_ERR_CUDA, "bundle_adjust launch failed");
-    FrameResult res;
-    if (!st) cudaMemcpyAsync(&res, E.P.results + slots[0], sizeof(FrameResult), cudaMemcpyDeviceToHost, E.stream);
     if (cudaStreamSynchronize(E.stream) != cudaSuccess && !st) st = fail(TBR_ERR_CUDA, "bundle_adjust failed");
-    E.blocks.release(fd.blk_off, fd.n_blocks);
-    E.free_slots.push_back(slots[0]);
+    release_frames(E, A.slots, A.devs);
     if (st) return st;
+    const FrameResult &res = E.h_results[0];
     for (int k = 0; k < 4; ++k) q[k] = res.q[k];
     for (int k = 0; k < 3; ++k) t[k] = res.t[k];
     if (stats) {
@@ -2100,7 +2077,8 @@ tbr_status tbr_batch_create(tbr_context *ctx, const tbr_frame_desc *frames, int3
     b->o = make_run_options(&ro, nullptr, ext);
     int64_t max_n = 0;
     std::vector<FrameDev> devs;
-    tbr_status st = admit_frames(E, fr, b->o, b->slots, max_n, &devs);
+    bool prepared = false;
+    tbr_status st = admit_frames(E, fr, b->o, b->slots, max_n, &prepared, &devs);
     for (size_t i = 0; i < b->slots.size() && i < devs.size(); ++i) {  // what batch_free releases
         b->ns.push_back(devs[i].n);
         b->blk_off.push_back(devs[i].blk_off);
@@ -2122,7 +2100,7 @@ tbr_status tbr_batch_create(tbr_context *ctx, const tbr_frame_desc *frames, int3
     b->Q.active = b->d_active;
     b->Q.n_active = n_frames;
     b->Q.prune = batch_prune(b);
-    E.launch_prep(b->Q, n_frames, max_n);
+    if (!prepared) E.launch_prep(b->Q, n_frames, max_n);
     // Snapshot the prepared frame states (AABB centre included).
     for (int i = 0; i < n_frames; ++i)
         cudaMemcpyAsync(b->d_init + i, E.P.frames + b->slots[i], sizeof(FrameDev), cudaMemcpyDeviceToDevice, E.stream);
@@ -2912,10 +2890,9 @@ tbr_status tbr_debug_score_samples(tbr_context *ctx, const double *points2D, con
     std::vector<int> slots;
     int64_t max_n = 0;
     TBR_CUDA(cudaSetDevice(E.device));
-    TBR_CUDA(cudaMemsetAsync(E.P.counters, 0, 8 * kCNum, E.stream));
-    tbr_status st = admit_frames(E, {fh}, o, slots, max_n);
+    bool prepared = false;
+    tbr_status st = admit_frames(E, {fh}, o, slots, max_n, &prepared, nullptr, false, true);
     if (st) return st;
-    E.launch_prep(1, max_n);
     E.P.prune = 0;  // every hypothesis's score is wanted
     k_plan<<<1, kMaxActive, 0, E.stream>>>(E.P);
     k_sample_p3p<<<E.p3p_grid, 128, 0, E.stream>>>(E.P);
