@@ -143,6 +143,15 @@ def _camera_K(camera):
     return K
 
 
+def _address(a):
+    """Address of an array's data (ctypes' buffer route is the cheapest one; read-only
+    and empty arrays go the long way)."""
+    try:
+        return C.addressof(C.c_char.from_buffer(a))
+    except (TypeError, ValueError, BufferError):
+        return a.ctypes.data
+
+
 def _f64(a, cols):
     a = np.ascontiguousarray(np.asarray(a, dtype=np.float64))
     if a.ndim != 2 or a.shape[1] != cols:
@@ -215,9 +224,9 @@ class Context:
         st = _lib.StatsC()
         with self._lock:
             check(_lib.lib().tbr_estimate_absolute_pose(
-                self._h, x.ctypes.data, X.ctypes.data, x.shape[0], K.ctypes.data, camera.width,
-                camera.height, C.byref(ro), C.byref(bo), C.byref(ext), q.ctypes.data, t.ctypes.data,
-                inl.ctypes.data, C.byref(st)))
+                self._h, _address(x), _address(X), x.shape[0], _address(K), camera.width,
+                camera.height, C.byref(ro), C.byref(bo), C.byref(ext), _address(q), _address(t),
+                _address(inl), C.byref(st)))
         stats = RansacStats_cuda(refinements=1 if not skip_refine else 0, iterations=st.samples,
                                  num_inliers=st.num_inliers, inlier_ratio=st.inlier_ratio,
                                  model_score=st.model_score, details=st.as_dict())
@@ -231,8 +240,8 @@ class Context:
         out = np.zeros(x.shape[0], np.uint8)
         cnt = C.c_int64()
         with self._lock:
-            check(_lib.lib().tbr_get_inliers(self._h, q.ctypes.data, t.ctypes.data, x.ctypes.data,
-                                             X.ctypes.data, x.shape[0], sq_threshold, out.ctypes.data,
+            check(_lib.lib().tbr_get_inliers(self._h, _address(q), _address(t), _address(x),
+                                             _address(X), x.shape[0], sq_threshold, _address(out),
                                              C.byref(cnt)))
         return out
 
@@ -251,9 +260,9 @@ class Context:
             w = np.ascontiguousarray(weights, np.float64)
         st = _lib.StatsC()
         with self._lock:
-            check(_lib.lib().tbr_bundle_adjust(self._h, x.ctypes.data, X.ctypes.data, x.shape[0], K.ctypes.data,
-                                               q.ctypes.data, t.ctypes.data, C.byref(bo),
-                                               w.ctypes.data if w is not None else None, C.byref(ext),
+            check(_lib.lib().tbr_bundle_adjust(self._h, _address(x), _address(X), x.shape[0], _address(K),
+                                               _address(q), _address(t), C.byref(bo),
+                                               _address(w) if w is not None else None, C.byref(ext),
                                                C.byref(st)))
         return CameraPose_cuda(q, t), st.as_dict()
 
@@ -336,6 +345,20 @@ _U64 = 0xFFFFFFFFFFFFFFFF
 _F64 = np.dtype(np.float64)
 
 
+def _frame_arrays(i, fr):
+    """Frame i's arrays as the C calls take them -- contiguous float64, kept alive by
+    the caller -- with their addresses and point count: (uv, xyz, &uv, &xyz, n)."""
+    u, x = fr.uv, fr.xyz
+    if type(u) is not np.ndarray or u.dtype != _F64 or not u.flags.c_contiguous:
+        u = np.ascontiguousarray(u, np.float64)
+    if type(x) is not np.ndarray or x.dtype != _F64 or not x.flags.c_contiguous:
+        x = np.ascontiguousarray(x, np.float64)
+    su, sx = u.shape, x.shape
+    if len(su) != 2 or su[1] != 2 or len(sx) != 2 or sx[1] != 3 or su[0] != sx[0]:
+        raise ValueError(f"frame {i}: uv must be (n, 2) and xyz (n, 3) with the same n")
+    return u, x, _address(u), _address(x), su[0]
+
+
 def _frame_descs(frames, seeds=None, max_reproj_error=0.0):
     """tbr_frame_desc entries for the frames' float64 arrays: (pointer for the C
     call, objects to keep alive until it returns). One pass over the frames
@@ -389,10 +412,14 @@ def _results(res, n, as_array=False):
     a = np.frombuffer(res, dtype=_RESULT_DTYPE, count=n)
     if as_array:
         return a
-    q, t, status = a["q"].copy(), a["t"].copy(), a["status"].tolist()
-    keys = ("q", "t", "status") + _STAT_NAMES
-    rows = a["stats"].tolist()
-    return [dict(zip(keys, (q[i], t[i], status[i]) + rows[i])) for i in range(n)]
+    return _rows(("q", "t", "status"), [list(a["q"].copy()), list(a["t"].copy()), a["status"].tolist()], a["stats"])
+
+
+def _rows(keys, columns, stats):
+    """One dict per result: the given columns, then the fields of the stats records,
+    converted a column at a time."""
+    keys += _STAT_NAMES
+    return [dict(zip(keys, row)) for row in zip(*columns, *(stats[k].tolist() for k in _STAT_NAMES))]
 
 
 class Batch:
@@ -655,11 +682,16 @@ class Server:
         check(_lib.lib().tbr_server_create(ctx.handle, C.byref(cfg), C.byref(h)))
         self._h = h
         self._buf = (_lib.ServerResultC * 1024)()
+        self._done = np.frombuffer(self._buf, dtype=np.dtype(_lib.ServerResultC))
         self._copy = copy
         self._keep = {}
 
     def submit(self, frame, seed: int | None = None, max_reproj_error: float = 0.0) -> int:
-        arr, keep = _frame_descs([frame], None if seed is None else [seed], max_reproj_error)
+        u, x, pu, px, n = _frame_arrays(0, frame)
+        K = np.asarray(frame.K, np.float64).reshape(4).tolist()
+        thr = max_reproj_error if max_reproj_error else getattr(frame, "threshold_px", 0.0)
+        arr = C.byref(_lib.FrameDescC(pu, px, n, (C.c_double * 4)(*K), int(frame.seed if seed is None else seed) & _U64, thr))
+        keep = (u, x)
         rid = C.c_uint64()
         if self._copy:
             check(_lib.lib().tbr_server_submit(self._h, arr, C.byref(rid)))
@@ -678,13 +710,15 @@ class Server:
         st = _lib.lib().tbr_server_poll(self._h, self._buf, min(max_results, 1024), C.byref(n))
         if st not in (0, 6):
             check(st)
-        out = []
-        for i in range(n.value):
-            r = self._buf[i]
-            self._keep.pop(r.request_id, None)
-            out.append({"id": r.request_id, "status": r.status, "q": np.array(r.q[:]), "t": np.array(r.t[:]),
-                        "latency_ms": r.submit_to_done_ms, **r.stats.as_dict()})
-        return out
+        if n.value == 0:
+            return []
+        a = self._done[:n.value]
+        ids = a["request_id"].tolist()
+        for i in ids:
+            self._keep.pop(i, None)
+        return _rows(("id", "status", "q", "t", "latency_ms"),
+                     [ids, a["status"].tolist(), list(a["q"].copy()), list(a["t"].copy()),
+                      a["submit_to_done_ms"].tolist()], a["stats"])
 
     def cancel(self, request_id: int):
         check(_lib.lib().tbr_server_cancel(self._h, request_id))

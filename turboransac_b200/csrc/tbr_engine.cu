@@ -17,10 +17,12 @@
 #include <cstdio>
 #include <cstring>
 #include <deque>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -168,6 +170,100 @@ static RunOptions make_run_options(const tbr_ransac_options *ro, const tbr_bundl
     return o;
 }
 
+// Host copies into pinned staging: a single core's memcpy bandwidth is well below
+// the link's, so an engine keeps up to 7 helper threads, started by the first copy
+// that wants them and joined with the engine. One run at a time (an engine's calls
+// are serialised by its lock; a server's engine belongs to its worker). Threads
+// started per call cost 15 us each, more than a copy of this size takes.
+class HelperThreads {
+   public:
+    ~HelperThreads() {
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            quit_ = true;
+        }
+        cv_.notify_all();
+        for (auto &t : th_) t.join();
+    }
+    // Runs `work` on every helper; the caller may run it too. finish() returns when
+    // all have returned from it.
+    void start(std::function<void()> work) {
+        if (th_.empty()) {
+            const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+            try {
+                for (unsigned t = 1; t < std::min(8u, hw); ++t) th_.emplace_back([this] { loop(); });
+            } catch (const std::system_error &) {  // no more threads to be had: fewer helpers, or none
+            }
+        }
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            work_ = std::move(work);
+            left_ = (int)th_.size();
+            ++run_;
+        }
+        cv_.notify_all();
+    }
+    void finish() {
+        std::unique_lock<std::mutex> lk(mu_);
+        done_.wait(lk, [&] { return left_ == 0; });
+        work_ = nullptr;
+    }
+
+   private:
+    void loop() {
+        uint64_t seen = 0;
+        for (;;) {
+            std::function<void()> w;
+            {
+                std::unique_lock<std::mutex> lk(mu_);
+                cv_.wait(lk, [&] { return quit_ || run_ != seen; });
+                if (quit_) return;
+                seen = run_;
+                w = work_;
+            }
+            w();
+            std::lock_guard<std::mutex> lk(mu_);
+            if (--left_ == 0) done_.notify_all();
+        }
+    }
+    std::vector<std::thread> th_;
+    std::mutex mu_;
+    std::condition_variable cv_, done_;
+    std::function<void()> work_;
+    uint64_t run_ = 0;
+    int left_ = 0;
+    bool quit_ = false;
+};
+
+struct CopyJob {
+    void *dst;
+    const void *src;
+    size_t bytes;
+};
+// From kCopyParallel bytes on with the helpers (they take about 30 us to wake; this
+// thread copies meanwhile), in pieces taken in turn.
+constexpr size_t kCopyParallel = 512u << 10, kCopyPiece = 64u << 10;
+static void parallel_copy(HelperThreads &helpers, const std::vector<CopyJob> &jobs) {
+    size_t total = 0;
+    for (auto &j : jobs) total += j.bytes;
+    if (total < kCopyParallel) {
+        for (auto &j : jobs) std::memcpy(j.dst, j.src, j.bytes);
+        return;
+    }
+    std::vector<CopyJob> pieces;
+    for (auto &j : jobs)
+        for (size_t o = 0; o < j.bytes; o += kCopyPiece)
+            pieces.push_back({(char *)j.dst + o, (const char *)j.src + o, std::min(kCopyPiece, j.bytes - o)});
+    std::atomic<size_t> next{0};
+    auto work = [&]() {
+        for (size_t k; (k = next.fetch_add(1)) < pieces.size();)
+            std::memcpy(pieces[k].dst, pieces[k].src, pieces[k].bytes);
+    };
+    helpers.start(work);
+    work();
+    helpers.finish();
+}
+
 // Whether a call's steps may score in two passes (k_prune): from a round of
 // kPruneMinPairs pairs over the frames that it can help. Each step then decides
 // by its own pairs (kPruneStepPairs); where none does, the two launches cost 6 us a
@@ -227,6 +323,7 @@ class Engine {
     cudaEvent_t ev_in = nullptr;
     char *d_ingest_first = nullptr;
     std::mutex mu;  // one call at a time per context
+    HelperThreads helpers;
 
     // Per-call buffers: h_stage (with its size and device alias),
     // d_ingest_first, h_counters, h_results, ev0, ev1 and ev_done above are
@@ -778,38 +875,6 @@ class Engine {
     }
 };
 
-// Host copies into pinned staging, split over threads when the batch is large
-// (a single core's memcpy bandwidth is well below the link's).
-struct CopyJob {
-    void *dst;
-    const void *src;
-    size_t bytes;
-};
-static void parallel_copy(const std::vector<CopyJob> &jobs) {
-    constexpr size_t kChunk = 1 << 20;
-    size_t total = 0;
-    for (auto &j : jobs) total += j.bytes;
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const int T = (int)std::min<size_t>(std::min(8u, hw), total / (4 * kChunk));
-    if (T <= 1) {
-        for (auto &j : jobs) std::memcpy(j.dst, j.src, j.bytes);
-        return;
-    }
-    std::vector<CopyJob> pieces;
-    for (auto &j : jobs)
-        for (size_t o = 0; o < j.bytes; o += kChunk)
-            pieces.push_back({(char *)j.dst + o, (const char *)j.src + o, std::min(kChunk, j.bytes - o)});
-    std::atomic<size_t> next{0};
-    auto work = [&]() {
-        for (size_t k; (k = next.fetch_add(1)) < pieces.size();)
-            std::memcpy(pieces[k].dst, pieces[k].src, pieces[k].bytes);
-    };
-    std::vector<std::thread> th;
-    for (int t = 1; t < T; ++t) th.emplace_back(work);
-    work();
-    for (auto &x : th) x.join();
-}
-
 // Admission in two halves. stage_frames (host only) takes slots and point
 // blocks and copies the frames into pinned staging; upload_staged enqueues the
 // device side. Frames whose point blocks are adjacent in the pool form one run;
@@ -922,7 +987,7 @@ static tbr_status stage_frames(Engine &E, const std::vector<FrameHost> &fr, cons
         A.hd[i] = A.devs[i];
         A.ha[i] = A.slots[i];
     }
-    if (copy) parallel_copy(jobs);
+    if (copy) parallel_copy(E.helpers, jobs);
     return TBR_OK;
 }
 
@@ -1108,13 +1173,9 @@ static tbr_status admit_host_frames(Engine &E, const std::vector<FrameHost> &fr,
             left[pieces[k].group].fetch_sub(1, std::memory_order_release);
         }
     };
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    std::vector<std::thread> th;
-    const size_t staged_bytes = pieces.size() * kPiece;
-    if (staged_bytes >= 4 * kPiece)
-        for (unsigned t = 0; t < std::min(8u, hw); ++t) th.emplace_back(work);
-    else
-        work();  // little to copy: this thread does it
+    const bool helped = pieces.size() >= 4;
+    if (helped) E.helpers.start(work);
+    else work();  // little to copy: this thread does it
     auto wait_group = [&](size_t g) {
         while (left[g].load(std::memory_order_acquire) > 0) std::this_thread::yield();
     };
@@ -1162,7 +1223,7 @@ static tbr_status admit_host_frames(Engine &E, const std::vector<FrameHost> &fr,
         return E.launch_graph((int)n, o.hr, stagger ? &sg : nullptr);
     };
     st = enqueue();
-    for (auto &x : th) x.join();
+    if (helped) E.helpers.finish();
     return st;
 }
 
@@ -1210,7 +1271,7 @@ static tbr_status admit_small(Engine &E, const std::vector<FrameHost> &fr, const
     const void **src = (const void **)((char *)E.h_stage + tab);
     std::vector<CopyJob> copies;
     for (size_t i = 0; i < n; ++i) stage_or_map(E, A, i, copies, src + 2 * i);
-    parallel_copy(copies);
+    parallel_copy(E.helpers, copies);
     k_admit_points<<<(int)n * kAdmitCtas, kAdmitThreads, 0, E.stream>>>(
         E.P, stage_alias(E, A.hd), stage_alias(E, A.ha), (const char *const *)stage_alias(E, src), E.d_active,
         clear ? 1 : 0);
@@ -1862,7 +1923,7 @@ tbr_status tbr_get_inliers(tbr_context *ctx, const double q[4], const double t[3
         dX = (const double *)mapped_address(X);
     if (!dx || !dX) {
         // x first, rounded up to 16 bytes (16 n always is)
-        parallel_copy({{h, x, 16 * (size_t)n}, {h + 16 * n, X, 24 * (size_t)n}});
+        parallel_copy(E.helpers, {{h, x, 16 * (size_t)n}, {h + 16 * n, X, 24 * (size_t)n}});
         dx = (const double *)stage_alias(E, h);
         dX = (const double *)stage_alias(E, h + 16 * n);
     }
@@ -1952,7 +2013,7 @@ tbr_status tbr_bundle_adjust(tbr_context *ctx, const double *x, const double *X,
     stage_or_map(E, A, 0, copies, src);
     double *hw = (double *)((char *)r0 + r0_bytes);
     if (weighted) copies.push_back({hw, weights, 8 * (size_t)n});
-    parallel_copy(copies);
+    parallel_copy(E.helpers, copies);
     E.P.n_active = 1;
     k_admit_lm<<<(int)std::min<int64_t>(32, (n + 511) / 512), 256, 0, E.stream>>>(
         E.P, stage_alias(E, A.hd), stage_alias(E, r0), A.slots[0], (const char *)src[0], (const char *)src[1],
