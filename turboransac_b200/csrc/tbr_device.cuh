@@ -304,45 +304,43 @@ __device__ int p3p_candidates(const d3 xin[3], const d3 Xin[3], P3PCtx &c, doubl
     c.X0 = X[0];
     for (int k = 0; k < 9; ++k) c.Mi[k] = Mi[k];
     c.a01 = a01, c.a02 = a02, c.a12 = a12, c.m01 = m01, c.m02 = m02, c.m12 = m12;
-    int n_sols = 0;
+    // Both lines, and both roots of each, side by side. A line is solved for the
+    // depth ratio tau of points 1 and 2 or of points 1 and 0, whichever divides by its
+    // larger coefficient: one flow with the coefficients chosen, since a warp has
+    // samples of either kind.
+    double dep0[4], dep1[4], dep2[4];
+    bool use[4];
+#pragma unroll
     for (int i = 0; i < 2; ++i) {
         const double p0 = pq[i][0], p1 = pq[i][1], p2 = pq[i][2];
-        if (fabs(p0) <= fabs(p1)) {
-            const double w0 = -p0 / p1, w1 = -p2 / p1;
-            const double ca = 1.0 / (w1 * w1 - b);
-            const double cb = 2.0 * (b * m12 - m02 * w1 + w0 * w1) * ca;
-            const double cc = (w0 * w0 - 2.0 * m02 * w0 - b + 1.0) * ca;
-            double taus[2];
-            if (!quad_roots(cb, cc, taus[0], taus[1])) continue;
-            for (int k = 0; k < 2; ++k) {
-                const double tau = taus[k];
-                if (tau <= 0) continue;
-                double d2 = sqrt(a12 / (tau * (tau - 2.0 * m12) + 1.0));
-                double d1 = tau * d2;
-                double d0 = (w0 * d2 + w1 * d1);
-                if (d0 < 0) continue;
-                dep[3 * n_sols] = d0, dep[3 * n_sols + 1] = d1, dep[3 * n_sols + 2] = d2;
-                ++n_sols;
-            }
-        } else {
-            const double w0 = -p1 / p0, w1 = -p2 / p0;
-            const double ca = 1.0 / (-a * w1 * w1 + 2.0 * a * m12 * w1 - a + 1.0);
-            const double cb = 2.0 * (a * m12 * w0 - m01 - a * w0 * w1) * ca;
-            const double cc = (1.0 - a * w0 * w0) * ca;
-            double taus[2];
-            if (!quad_roots(cb, cc, taus[0], taus[1])) continue;
-            for (int k = 0; k < 2; ++k) {
-                const double tau = taus[k];
-                if (tau <= 0.0) continue;
-                double d0 = sqrt(a01 / (tau * (tau - 2.0 * m01) + 1.0));
-                double d1 = tau * d0;
-                double d2 = w0 * d0 + w1 * d1;
-                if (d2 < 0.0) continue;
-                dep[3 * n_sols] = d0, dep[3 * n_sols + 1] = d1, dep[3 * n_sols + 2] = d2;
-                ++n_sols;
-            }
+        const bool first = fabs(p0) <= fabs(p1);
+        const double pd = first ? p1 : p0;
+        const double w0 = (first ? -p0 : -p1) / pd, w1 = -p2 / pd;
+        const double ca = 1.0 / (first ? w1 * w1 - b : -a * w1 * w1 + 2.0 * a * m12 * w1 - a + 1.0);
+        const double cb = 2.0 * (first ? b * m12 - m02 * w1 + w0 * w1 : a * m12 * w0 - m01 - a * w0 * w1) * ca;
+        const double cc = (first ? w0 * w0 - 2.0 * m02 * w0 - b + 1.0 : 1.0 - a * w0 * w0) * ca;
+        double taus[2];
+        const bool real = quad_roots(cb, cc, taus[0], taus[1]);
+        const double aa = first ? a12 : a01, mm = first ? m12 : m01;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const double tau = taus[k];
+            const double d = sqrt(aa / (tau * (tau - 2.0 * mm) + 1.0));
+            const double d1 = tau * d;
+            const double e = w0 * d + w1 * d1;  // the third depth
+            dep0[2 * i + k] = first ? e : d;
+            dep1[2 * i + k] = d1;
+            dep2[2 * i + k] = first ? d : e;
+            use[2 * i + k] = real && !(tau <= 0.0) && !(e < 0.0);
         }
-        if (n_sols > 0 && G) break;
+    }
+    int n_sols = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j == 2 && n_sols > 0 && G) break;
+        if (!use[j]) continue;
+        dep[3 * n_sols] = dep0[j], dep[3 * n_sols + 1] = dep1[j], dep[3 * n_sols + 2] = dep2[j];
+        ++n_sols;
     }
     return n_sols;
 }

