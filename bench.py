@@ -825,8 +825,8 @@ def stored_traffic(kernel: str, frames):
         return int(k["bytes_per_staged_point"] * pts), (
             f"not measured in this run: first engine step's launch (all frames active), ncu "
             f"dram__bytes_read.sum + dram__bytes_write.sum of the 64-frame case captured {k['captured']} "
-            f"({k['bytes_per_staged_point']:.1f} B per staged point: each point's 40-byte record and each "
-            f"hypothesis read once) x {pts} staged points; {k['summary']}"), k.get("pipes_first_launch")
+            f"({k['bytes_per_staged_point']:.1f} B per staged point: the first pass reads a prefix of each frame's "
+            f"points and each hypothesis once) x {pts} staged points; {k['summary']}"), k.get("pipes_first_launch")
     except Exception:
         return None, f"no stored ncu capture of {kernel} on this workload", None
 

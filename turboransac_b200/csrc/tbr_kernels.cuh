@@ -1045,8 +1045,8 @@ __global__ void __launch_bounds__(kScoreWarps * 32) k_score(Pools P) {
 
 // ------------------------------------------------ tensor-core scoring --
 // The same filter with the projection on the 5th-generation tensor cores: for
-// a block of 128 hypotheses and a tile of 32 points, three pairs of
-// tcgen05.mma (kind::tf32, M = 128 hypotheses, N = 32 points, K = 16 in two
+// a block of 128 hypotheses and a tile of 64 points, three pairs of
+// tcgen05.mma (kind::tf32, M = 128 hypotheses, N = 64 points, K = 16 in two
 // steps of 8) write every z2, z0 and z1 of the tile into tensor memory, and the
 // epilogue -- one thread per hypothesis -- does the reciprocal, the residuals,
 // the saturating r^2 and its own hypothesis's sum. TF32 keeps 11 significant
