@@ -122,3 +122,26 @@ def test_mixed_host_arrays(ctx):
         np.testing.assert_array_equal(r["q"], pose.q)
         np.testing.assert_array_equal(r["t"], pose.t)
         np.testing.assert_array_equal(r["inliers"].astype(bool), np.asarray(one).astype(bool))
+
+
+ONE_PROCESSOR = """
+import os
+os.sched_setaffinity(0, {min(os.sched_getaffinity(0))})
+import numpy as np
+from turboransac_b200 import Context, RansacOptions_cuda, estimate_batch, scenes
+ctx = Context(0, 1 << 30)
+frames = [scenes.make_frame(30000, 0.6, 0.5, 50 + i) for i in range(%d)]
+r = estimate_batch(ctx, frames, RansacOptions_cuda(max_iterations=64, max_reproj_error=4.0))
+assert len(r) == len(frames) and all(x["num_inliers"] > 15000 for x in r)
+"""
+
+
+@pytest.mark.parametrize("frames", [1, 2, 5, 16])
+def test_host_copies_without_helper_threads(frames):
+    """A process bound to one processor has no helpers to copy for it: one frame, a
+    small batch, an ingested one (6 MB) and one whose ingestion overlaps its run (19 MB)."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", ONE_PROCESSOR % frames], cwd=root, check=True, timeout=120)

@@ -186,8 +186,9 @@ class HelperThreads {
         for (auto &t : th_) t.join();
     }
     // Runs `work` on every helper; the caller may run it too. finish() returns when
-    // all have returned from it.
-    void start(std::function<void()> work) {
+    // all have returned from it. False: there is no helper (one processor, or no
+    // threads to be had), and nothing runs but what the caller does.
+    bool start(std::function<void()> work) {
         if (th_.empty()) {
             const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
             try {
@@ -195,6 +196,7 @@ class HelperThreads {
             } catch (const std::system_error &) {  // no more threads to be had: fewer helpers, or none
             }
         }
+        if (th_.empty()) return false;
         {
             std::lock_guard<std::mutex> lk(mu_);
             work_ = std::move(work);
@@ -202,6 +204,7 @@ class HelperThreads {
             ++run_;
         }
         cv_.notify_all();
+        return true;
     }
     void finish() {
         std::unique_lock<std::mutex> lk(mu_);
@@ -1173,9 +1176,8 @@ static tbr_status admit_host_frames(Engine &E, const std::vector<FrameHost> &fr,
             left[pieces[k].group].fetch_sub(1, std::memory_order_release);
         }
     };
-    const bool helped = pieces.size() >= 4;
-    if (helped) E.helpers.start(work);
-    else work();  // little to copy: this thread does it
+    const bool helped = pieces.size() >= 4 && E.helpers.start(work);
+    if (!helped) work();  // little to copy, or no helpers: this thread does it
     auto wait_group = [&](size_t g) {
         while (left[g].load(std::memory_order_acquire) > 0) std::this_thread::yield();
     };
