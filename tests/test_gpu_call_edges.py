@@ -145,3 +145,39 @@ def test_host_copies_without_helper_threads(frames):
     import sys
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     subprocess.run([sys.executable, "-c", ONE_PROCESSOR % frames], cwd=root, check=True, timeout=120)
+
+
+def off_boundary(a):
+    """Page-locked, 4 bytes off an 8-byte boundary (a view into packed records, say)."""
+    import torch
+    raw = torch.empty(a.nbytes + 8, dtype=torch.uint8, pin_memory=True).numpy()
+    out = raw[4:4 + a.nbytes].view(np.float64).reshape(a.shape)
+    out[:] = a
+    assert out.ctypes.data % 8 == 4
+    return out
+
+
+@pytest.mark.parametrize("frames", [1, 3, 6])
+def test_page_locked_arrays_off_their_boundary(ctx, oracle, frames):
+    """Read from a staging copy, not in place: a frame alone, a small batch and an
+    ingested one (7 MB), a pose's mask and a bundle adjustment."""
+    import copy
+    fr = [scenes.make_frame(30000, 0.6, 0.5, 70 + i) for i in range(frames)]
+    odd = []
+    for f in fr:
+        g = copy.copy(f)
+        g.uv, g.xyz = off_boundary(f.uv), off_boundary(f.xyz)
+        odd.append(g)
+    for a, b in zip(estimate_batch(ctx, fr, options()), estimate_batch(ctx, odd, options())):
+        np.testing.assert_array_equal(a["q"], b["q"])
+        np.testing.assert_array_equal(a["t"], b["t"])
+    f = fr[0]
+    xn = np.ascontiguousarray((f.uv - [f.K[2], f.K[3]]) / [f.K[0], f.K[1]])
+    pose = CameraPose_cuda(oracle.rotmat_to_quat(f.R_gt), f.t_gt)
+    thr = 16.0 / (0.5 * (f.K[0] + f.K[1])) ** 2
+    np.testing.assert_array_equal(ctx.get_inliers(pose, off_boundary(xn), odd[0].xyz, thr),
+                                  ctx.get_inliers(pose, xn, f.xyz, thr))
+    p0, _ = ctx.bundle_adjust(f.uv, f.xyz, cam_of(f), pose, BundleOptions_cuda(loss_scale=1.0))
+    p1, _ = ctx.bundle_adjust(odd[0].uv, odd[0].xyz, cam_of(f), pose, BundleOptions_cuda(loss_scale=1.0))
+    np.testing.assert_array_equal(p0.q, p1.q)
+    np.testing.assert_array_equal(p0.t, p1.t)

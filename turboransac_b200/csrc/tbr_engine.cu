@@ -1056,14 +1056,20 @@ static const int64_t *put_table(Engine &E, char *h, size_t &off, const std::vect
     off += (bytes + 15) & ~size_t(15);
     return d;
 }
-// Device address of page-locked host memory (nullptr for pageable memory).
-static const void *mapped_address(const void *p) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
+// Device address of page-locked host memory that kernels can read in place: page-locked
+// from the first byte to the last and on an 8-byte boundary (nullptr otherwise).
+static const void *mapped_address(const void *p, size_t bytes) {
+    if (reinterpret_cast<uintptr_t>(p) & 7) return nullptr;
+    const char *ends[2] = {(const char *)p, (const char *)p + (bytes - 1)}, *dev[2];
+    for (int k = 0; k < 2; ++k) {
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, ends[k]) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (at.type != cudaMemoryTypeHost || !(dev[k] = (const char *)at.devicePointer)) return nullptr;
     }
-    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+    return dev[1] - dev[0] == (ptrdiff_t)(bytes - 1) ? dev[0] : nullptr;
 }
 
 // Host-buffer admission by zero-copy ingestion: every frame's arrays are read
@@ -1115,8 +1121,8 @@ static tbr_status admit_host_frames(Engine &E, const std::vector<FrameHost> &fr,
     size_t total = 0;
     for (size_t k = 0; k < n; ++k) {
         total += (fb[k] = A.jobs[2 * k].bytes + A.jobs[2 * k + 1].bytes);
-        su[k] = mapped_address(fr[k].uv);
-        sx[k] = su[k] ? mapped_address(fr[k].xyz) : nullptr;
+        su[k] = mapped_address(fr[k].uv, 16 * (size_t)fr[k].n);
+        sx[k] = su[k] ? mapped_address(fr[k].xyz, 24 * (size_t)fr[k].n) : nullptr;
         if (!su[k] || !sx[k]) {
             staged[k] = 1;
             su[k] = (const char *)E.d_stage_alias + ((const char *)A.jobs[2 * k].dst - (const char *)E.h_stage);
@@ -1241,7 +1247,8 @@ constexpr size_t kMappedQueryBytes = 128u << 10;
 static void stage_or_map(Engine &E, const StagedAdmission &A, size_t i, std::vector<CopyJob> &copies, const void **src) {
     const CopyJob &u = A.jobs[2 * i], &x = A.jobs[2 * i + 1];
     const void *mu = nullptr, *mx = nullptr;
-    if (u.bytes + x.bytes >= kMappedQueryBytes && (mu = mapped_address(u.src))) mx = mapped_address(x.src);
+    if (u.bytes + x.bytes >= kMappedQueryBytes && (mu = mapped_address(u.src, u.bytes)))
+        mx = mapped_address(x.src, x.bytes);
     if (mu && mx) {
         src[0] = mu;
         src[1] = mx;
@@ -1921,8 +1928,8 @@ tbr_status tbr_get_inliers(tbr_context *ctx, const double q[4], const double t[3
     if (!E.d_stage_alias) return fail(TBR_ERR_CUDA, "staging buffer has no device address");
     char *h = (char *)E.h_stage;
     const double *dx = nullptr, *dX = nullptr;
-    if (40 * (size_t)n >= kMappedQueryBytes && (dx = (const double *)mapped_address(x)))
-        dX = (const double *)mapped_address(X);
+    if (40 * (size_t)n >= kMappedQueryBytes && (dx = (const double *)mapped_address(x, 16 * (size_t)n)))
+        dX = (const double *)mapped_address(X, 24 * (size_t)n);
     if (!dx || !dX) {
         // x first, rounded up to 16 bytes (16 n always is)
         parallel_copy(E.helpers, {{h, x, 16 * (size_t)n}, {h + 16 * n, X, 24 * (size_t)n}});
