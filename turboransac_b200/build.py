@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 SRC = os.path.join(HERE, "csrc", "tbr_engine.cu")
 OUT = os.path.join(HERE, "libtbr.so")
-DEPS = [os.path.join(HERE, "csrc", f) for f in ("tbr_engine.cu", "tbr_kernels.cuh", "tbr_device.cuh")] + [
+DEPS = [os.path.join(HERE, "csrc", f) for f in ("tbr_engine.cu", "tbr_host.h", "tbr_kernels.cuh", "tbr_device.cuh")] + [
     os.path.join(ROOT, "include", "tbr.h")]
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

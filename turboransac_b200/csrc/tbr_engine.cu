@@ -7,6 +7,7 @@
 // and synchronises the whole device 4 times per round; here nothing is
 // allocated per call and a round needs no host round-trip.
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,6 +29,7 @@
 #include <vector>
 
 #include "../../include/tbr.h"
+#include "tbr_host.h"
 #include "tbr_kernels.cuh"
 
 namespace tbr {
@@ -1056,20 +1058,35 @@ static const int64_t *put_table(Engine &E, char *h, size_t &off, const std::vect
     off += (bytes + 15) & ~size_t(15);
     return d;
 }
-// Device address of page-locked host memory that kernels can read in place: page-locked
-// from the first byte to the last and on an 8-byte boundary (nullptr otherwise).
-static const void *mapped_address(const void *p, size_t bytes) {
-    if (reinterpret_cast<uintptr_t>(p) & 7) return nullptr;
-    const char *ends[2] = {(const char *)p, (const char *)p + (bytes - 1)}, *dev[2];
-    for (int k = 0; k < 2; ++k) {
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, ends[k]) != cudaSuccess) {
+// Device address of page-locked host memory that kernels can read in place: on an
+// 8-byte boundary and within one page-locked range from the first byte to the last
+// (nullptr otherwise). The driver is asked for the range: two ends that are page-locked
+// may belong to two registrations with a hole between them.
+using PointerQuery = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+static PointerQuery pointer_query() {
+    static const PointerQuery f = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &p, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
-            return nullptr;
+            p = nullptr;
         }
-        if (at.type != cudaMemoryTypeHost || !(dev[k] = (const char *)at.devicePointer)) return nullptr;
-    }
-    return dev[1] - dev[0] == (ptrdiff_t)(bytes - 1) ? dev[0] : nullptr;
+        return (PointerQuery)p;
+    }();
+    return f;
+}
+static const void *mapped_address(const void *p, size_t bytes) {
+    const PointerQuery query = pointer_query();
+    if (!query || (reinterpret_cast<uintptr_t>(p) & 7)) return nullptr;
+    unsigned type = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute at[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *out[4] = {&type, &dev, &start, &size};
+    if (query(4, at, out, (CUdeviceptr)p) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || !dev) return nullptr;
+    return range_holds(start, size, (CUdeviceptr)p, bytes) ? (const void *)dev : nullptr;
 }
 
 // Host-buffer admission by zero-copy ingestion: every frame's arrays are read
