@@ -427,11 +427,11 @@ class Engine {
                              3 * (kMaxActive + 1) * 8 + 4096 * 8;
         if (budget < fixed + (64ull << 20)) return fail(TBR_ERR_INVALID_ARG, "workspace too small");
         const size_t rest = budget - fixed;
-        const size_t per_hyp = 96 + 48 + 8 + 4 + 4 * 32 + 4 + 4;
+        const size_t per_hyp = 96 + 48 + 8 + 4 + 4 * 32 + 4;
         P.max_hyps = (int64_t)(rest * 0.3 / per_hyp);
         P.max_hyps = std::max<int64_t>(P.max_hyps, 4096);
         P.max_parts = P.max_hyps * 32;
-        P.max_hb = P.max_hyps / 32 + kMaxActive;
+        P.max_hb = P.max_hyps / 64 + kMaxActive;  // blocks of 64 hypotheses (the narrowest FP32 shape) or 128
         const size_t per_block = (size_t)kSub * (16 + 24 + 16 + 1 + 16 + 24 + 8 + 8) + kBlockBytes;
         max_blocks = (int64_t)((rest - (size_t)(P.max_hyps * per_hyp) - P.max_hb * 4) / per_block) - 1;
         if (max_blocks < 64) return fail(TBR_ERR_INVALID_ARG, "workspace too small for points");
@@ -465,7 +465,6 @@ class Engine {
         add((void **)&P.hId, 8 * P.max_hyps);
         add((void **)&P.hS32, 4 * P.max_hyps);
         add((void **)&P.part, 4 * P.max_parts);
-        add((void **)&P.surv, 4 * P.max_hyps);
         add((void **)&P.hb_arrive, 4 * P.max_hb);
         add((void **)&P.cHyp, 4 * (size_t)P.cand_cap);
         add((void **)&P.cS64, 8 * (size_t)P.cand_cap);
@@ -484,6 +483,7 @@ class Engine {
             *p.first = cur;
             cur += (p.second + 255) & ~size_t(255);
         }
+        P.surv = (int32_t *)P.dbg_counts;  // no call both scores in two passes and counts for debugging
         P.active = d_active;
         P.num_sms = num_sms;
         P.lm_cluster_min = kLMClusterMin;

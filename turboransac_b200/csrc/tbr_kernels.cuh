@@ -185,7 +185,7 @@ struct Pools {
     int64_t *hId;
     float *hS32;
     float *part;
-    int32_t *surv;       // two-pass scoring: a frame's hypotheses left, from its hyp_base
+    int32_t *surv;       // two-pass scoring: a frame's hypotheses left, from its hyp_base (shares dbg_counts)
     int32_t prune;       // 1: the step has a second scoring pass
     int32_t pad0;
     unsigned *hb_arrive;
