@@ -567,10 +567,6 @@ class Engine {
         f.focal = 0.5 * (fh.K[0] + fh.K[1]);          // Camera_cuda::focal, camera.cuh:64-67
         f.tau = fh.max_reproj_error / f.focal;        // entry.cu:48-49
         f.sq_thr = f.tau * f.tau;                     // turbo_ransac.cu:34
-        for (int k = 0; k < 3; ++k) {
-            f.bmin[k] = ~0ull;
-            f.bmax[k] = 0ull;
-        }
         f.B = o.B;
         f.max_total = o.max_total;
         f.min_samples = o.min_samples;
@@ -597,6 +593,7 @@ class Engine {
         f.best_score = DBL_MAX;
         f.best_sample = -1;
         f.best_sol = -1;
+        f.residual_unit = (float)(kResidualError / f.tau);
         return f;
     }
 
@@ -690,7 +687,6 @@ class Engine {
 
     void launch_prep(const Pools &Q, int n_active, int64_t max_n, cudaStream_t st) {
         const int bx = (int)std::min<int64_t>(64, std::max<int64_t>(1, (max_n + 1023) / 1024));
-        k_prep_bounds<<<dim3(bx, n_active), 256, 0, st>>>(Q);
         k_prep_pack<<<dim3(bx, n_active), 256, 0, st>>>(Q);
         k_prosac_table<<<n_active, 1024, 0, st>>>(Q);
     }
@@ -2188,7 +2184,7 @@ tbr_status tbr_batch_create(tbr_context *ctx, const tbr_frame_desc *frames, int3
     b->Q.n_active = n_frames;
     b->Q.prune = batch_prune(b);
     if (!prepared) E.launch_prep(b->Q, n_frames, max_n);
-    // Snapshot the prepared frame states (AABB centre included).
+    // Snapshot the prepared frame states (centre included).
     for (int i = 0; i < n_frames; ++i)
         cudaMemcpyAsync(b->d_init + i, E.P.frames + b->slots[i], sizeof(FrameDev), cudaMemcpyDeviceToDevice, E.stream);
     if (cudaStreamSynchronize(E.stream) != cudaSuccess) {
@@ -2671,7 +2667,7 @@ static tbr_status server_step(tbr_server *s) {
     if (!A.slots.empty()) {
         tbr_status st = upload_staged(E, A);
         if (st) return st;
-        // upload_staged wrote the new slots to d_active; prepare them (AABB, packing).
+        // upload_staged wrote the new slots to d_active; prepare them (centre, packing).
         TBR_CUDA(cudaMemcpyAsync(s->d_prep, E.d_active, 4 * A.slots.size(), cudaMemcpyDeviceToDevice, E.stream));
         Pools Q = E.P;
         Q.active = s->d_prep;

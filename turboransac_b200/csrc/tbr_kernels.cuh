@@ -113,7 +113,6 @@ struct __align__(16) FrameDev {
     double K[4];
     double focal, tau, sq_thr;
     double centre[3];
-    unsigned long long bmin[3], bmax[3];
     int64_t B;
     int64_t max_total;
     int64_t min_samples;  // no stop before this many samples (honoured min_iterations; else 0)
@@ -151,11 +150,16 @@ struct __align__(16) FrameDev {
                              // hypotheses left for the second (Pools::surv)
     int32_t cand_count, n_rchunks;
     int64_t rchunk, cand_base;
+    // round_min starts a 128-byte line in the first slot: beside the fields above, which
+    // every item reads, its atomics made scoring 6 % slower (100000 samples of 1537 points,
+    // one frame: 146 -> 155 us).
+    int64_t pad_line[6];
     unsigned long long round_min[kMaxRoundsPerStep];
     // ---- LM ----
     int64_t num_inliers;
     int64_t lm_epoch;  // engine step in which RANSAC finished
-    int32_t lm_force_cluster, pad9;  // bundle_adjust path: always the cluster LM
+    int32_t lm_force_cluster;  // bundle_adjust path: always the cluster LM
+    float residual_unit;       // the FP32 filter's residual error (filter_error), kResidualError / tau
 };
 
 struct Pools {
@@ -314,36 +318,43 @@ __device__ __forceinline__ int round_of(const FrameDev &f, int64_t id) {
 }
 
 // ----------------------------------------------------------- admission -----
-// AABB of the frame's world points (ordered-integer atomics: order independent).
-__global__ void k_prep_bounds(Pools P) {
-    const int a = blockIdx.y;
-    if (a >= P.n_active) return;
-    FrameDev &f = P.frames[P.active[a]];
-    const int64_t base = f.blk_off * kSub;
-    double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < f.n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const double v0 = P.X64[3 * (base + i)], v1 = P.X64[3 * (base + i) + 1], v2 = P.X64[3 * (base + i) + 2];
-        if (!(isfinite(v0) && isfinite(v1) && isfinite(v2))) continue;  // staged as an outlier
-        const double v[3] = {v0, v1, v2};
+// Centre of a frame's world points, from which the FP32 filter holds them: in each
+// coordinate the lower median of up to 64 points spread over the frame's order (finite
+// ones; 0 without any). A median stays among the points where outliers, however far,
+// are fewer than half. The middle of their box goes where the farthest ones lie: with
+// one point in a hundred 100 m away from a room of 5000 points at 95 % inliers, FP32
+// scores were off by up to 0.58, now 0.03, as without. Every CTA finds it for itself
+// (192 threads).
+constexpr int kCentrePts = 64;
+__device__ __forceinline__ void frame_centre(const double *X, int64_t n, double (&cc)[3]) {
+    __shared__ double smp[3][kCentrePts], mid[3];
+    const int t = threadIdx.x;
+    if (t < kCentrePts) {
+        const int64_t i = n < kCentrePts ? t : t * n / kCentrePts;
+        double v[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            lo[k] = fmin(lo[k], v[k]);
-            hi[k] = fmax(hi[k], v[k]);
-        }
+        for (int k = 0; k < 3; ++k) v[k] = i < n ? __ldcg(X + 3 * i + k) : INFINITY;
+        const bool ok = isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) smp[k][t] = ok ? v[k] : INFINITY;
+        if (t < 3) mid[t] = 0.0;
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[k] = fmin(lo[k], __shfl_down_sync(0xffffffffu, lo[k], o));
-            hi[k] = fmax(hi[k], __shfl_down_sync(0xffffffffu, hi[k], o));
+    __syncthreads();
+    if (t < 3 * kCentrePts) {
+        const int k = t / kCentrePts, j = t % kCentrePts;
+        const double v = smp[k][j];
+        int rank = 0, m = 0;
+#pragma unroll 8
+        for (int q = 0; q < kCentrePts; ++q) {
+            const double u = smp[k][q];
+            rank += u < v || (u == v && q < j) ? 1 : 0;
+            m += isfinite(u) ? 1 : 0;
         }
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(&f.bmin[k], dbl_to_ordered(lo[k]));
-            atomicMax(&f.bmax[k], dbl_to_ordered(hi[k]));
-        }
+        if (isfinite(v) && rank == (m - 1) / 2) mid[k] = v;
     }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) cc[k] = mid[k];
 }
 
 // The FP32 filter's view of a point: the centred world point and -x/tau, -y/tau.
@@ -402,19 +413,13 @@ __device__ __forceinline__ void pack_point(const Pools &P, const FrameDev &f, in
         for (int k = 0; k < 5; ++k) blk[k * kSub + j] = make_float2(v[k], v[k]);
     }
 }
-__device__ __forceinline__ void box_centre(const unsigned long long *bmin, const unsigned long long *bmax, double (&cc)[3]) {
-    for (int k = 0; k < 3; ++k) {  // no finite point: centre 0
-        cc[k] = 0.5 * (ordered_to_dbl(bmin[k]) + ordered_to_dbl(bmax[k]));
-        if (!isfinite(cc[k])) cc[k] = 0.0;
-    }
-}
 __global__ void k_prep_pack(Pools P) {
     const int a = blockIdx.y;
     if (a >= P.n_active) return;
     FrameDev &f = P.frames[P.active[a]];
     const int64_t base = f.blk_off * kSub;
     double cc[3];
-    box_centre(f.bmin, f.bmax, cc);
+    frame_centre(P.X64 + 3 * base, f.n, cc);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         f.centre[0] = cc[0];
         f.centre[1] = cc[1];
@@ -699,6 +704,29 @@ __global__ void __launch_bounds__(128) k_sample_p3p(Pools P) {
     }
 }
 
+// ------------------------------------------------- the filter's error -----
+// Bound on |s32 - s64| for a score s near the running best's, in tau^2 units. Two
+// parts: the sums' rounding, s/65536 + 1/4, and the rounding of each residual, of the
+// order of 2^-24 (|X| + |t|) / (z tau) for a point at depth z, X and t from the
+// frame's centre. Part of the second is the same for every point of a hypothesis (the
+// rounding of its rows), so by Cauchy-Schwarz over the inliers it moves the score by
+// up to 2 d sqrt(n s) for a residual error d, and by less where there are few
+// inliers: their gain is n - s. d = kResidualError / (2 tau) held over thresholds of 0.1
+// to 12 px, focal lengths of 200 to 2000, 2000 to 200000 points, 10 to 95 % inliers,
+// thin, flat and deep scenes (depths over two decades) and outliers up to 1 km away:
+// in 915 frames, the 150 best hypotheses of each, the largest error was 0.88 of the
+// bound. At 4 px and f = 525 the first part is the larger one up to 15000 points.
+constexpr double kResidualError = 1.5 * 0x1p-22;
+__device__ __forceinline__ float filter_error(const FrameDev &f, float s) {
+    const float n = (float)f.n;
+    return fmaxf(s * (1.0f / 65536.0f) + 0.25f, f.residual_unit * fminf(sqrtf(n * s), n - s));
+}
+// What k_prune's bound leaves above the running best T: more than the candidate band
+// (k_select) and the error of a hypothesis's own score.
+__device__ __forceinline__ float prune_margin(const FrameDev &f, float T) {
+    return fmaxf(T * (1.0f / 2048.0f) + 2.0f, 5.0f * filter_error(f, T));
+}
+
 // ------------------------------------------------------------ scoring -----
 // Staging blocks of a frame's first scoring pass; 0: one pass over all of them.
 // With a best model from earlier steps the prefix is long enough that a
@@ -711,7 +739,8 @@ __device__ __forceinline__ int first_pass_blocks(const FrameDev &f) {
     const float n = (float)f.n;
     float m = fminf(fmaxf(0.25f * n, 512.0f), 1024.0f);
     if (f.found) {
-        const float mu = 1.0f - (float)(f.best_score / f.sq_thr) * (1.0f + 1.0f / 2048.0f) / n - 2.0f / n;
+        const float T = (float)(f.best_score / f.sq_thr);
+        const float mu = 1.0f - (T + prune_margin(f, T)) / n;
         if (!(mu > 0.0f)) return 0;
         m = fmaxf(512.0f, (4.0f / 3.0f) * kPruneLog / mu);
     }
@@ -1421,7 +1450,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) k_score_tc(Pools P, int p
 // full scores -- computed here -- of this and earlier rounds' leaders after
 // the first pass. A hypothesis matters only if its score is inside the candidate
 // band of the running best (k_select), i.e. its mean gain is at least
-// mu = 1 - (T + T/2048 + 2) / n, the band taken wide enough for both FP32 sums. It
+// mu = 1 - (T + prune_margin) / n, the band taken wide enough for both FP32 sums. It
 // is dropped when its sample mean has KL(x || mu) >= kPruneLog / m: a hypothesis
 // that matters is dropped with probability < exp(-46) < 2^-64. The others,
 // typically a few percent, are scored on the remaining points.
@@ -1501,9 +1530,9 @@ __global__ void __launch_bounds__(1024) k_prune(Pools P) {
         }
         // The sample sum from which a hypothesis is dropped: the largest x with
         // m KL(x || mu) >= kPruneLog by bisection (12 steps, the safe end), with a
-        // margin for the FP32 sum.
+        // margin for the FP32 sum and its residuals.
         if (w == 0) {
-            const float mu = 1.0f - T * (1.0f + 1.0f / 2048.0f) / n - 2.0f / n;
+            const float mu = 1.0f - (T + prune_margin(f, T)) / n;
             float c = inf;
             if (mu > 0.0f && m * bernoulli_kl(0.0f, mu) >= kPruneLog) {
                 float lo = 0.0f, hi = mu;
@@ -1511,7 +1540,8 @@ __global__ void __launch_bounds__(1024) k_prune(Pools P) {
                     const float x = 0.5f * (lo + hi);
                     if (m * bernoulli_kl(x, mu) >= kPruneLog) lo = x; else hi = x;
                 }
-                c = m * (1.0f - lo) + m * 2e-5f;
+                c = m * (1.0f - lo);
+                c += fmaxf(m * 2e-5f, f.residual_unit * sqrtf(m * c));
             }
             for (int r = lane; r < R; r += 32) cut[r] = r >= from ? c : inf;
         }
@@ -1557,14 +1587,14 @@ __global__ void __launch_bounds__(1024) k_prune(Pools P) {
 // ---------------------------------------------------------- candidates -----
 // Candidates for the exact FP64 re-rank: every hypothesis whose FP32 score s
 // lies within a band of the running minimum thr of its round (over this
-// step's rounds so far and the best of earlier steps), s <= thr + thr/16384 + 1
-// (scores in tau^2 units). The FP32 score of a hypothesis is within 1e-5 of
-// its FP64 score relative (tested), so the FP64 best of every round that can
-// change the running best -- including every exact tie -- lies inside the
-// safe band thr + thr/32768 + 1/2, twice that error on both sides with an
-// absolute margin, and the candidate band is twice the safe band (a band of thr/4096
-// + 1 re-ranked 4159 candidates on a frame of 50000 points at 8 % inliers, 1.06 ms,
-// this one 71, 0.08 ms, with the same selection). It is never narrowed. When more than kMaxCandFrame hypotheses fall inside it:
+// step's rounds so far and the best of earlier steps), s <= thr + 4 E(thr) (scores in
+// tau^2 units; E is filter_error's bound). The FP64 best of every round that can
+// change the running best -- including every exact tie -- lies inside the safe band
+// thr + 2 E, an error of E on both sides, and the candidate band is twice the safe
+// band: thr + thr/16384 + 1 where the sums' rounding is the larger part of E (a band of
+// thr/4096 + 1 re-ranked 4159 candidates on a frame of 50000 points at 8 % inliers,
+// 1.06 ms, this one 71, 0.08 ms, with the same selection). It is never narrowed. When more
+// than kMaxCandFrame hypotheses fall inside it:
 //   * a step of several rounds (forced mode: more than kSplitSamples samples)
 //     is redone: the frame's later steps are limited to the rounds that the
 //     step's candidate rate leaves room for (half the cap, and fewer rounds
@@ -1586,8 +1616,6 @@ __device__ __forceinline__ unsigned long long cand_key(float s, float t, float i
     const float u = fmaxf((s - t) * inv_safe, 0.0f);
     return ((unsigned long long)__float_as_uint(u) << 32) | (unsigned long long)(uint32_t)(id - 4 * first);
 }
-
-__device__ __forceinline__ float cand_limit(float t) { return t + (t * (1.0f / 16384.0f) + 1.0f); }
 
 // Work items of the re-rank: (frame, group of candidates, point chunk).
 __device__ __forceinline__ void rescore_plan(const Pools &P) {
@@ -1628,7 +1656,7 @@ __device__ __forceinline__ void rescore_plan(const Pools &P) {
 
 // One CTA per frame; the launch's last CTA to finish plans the re-rank.
 __device__ __forceinline__ void select_frame(const Pools &P) {
-    __shared__ float thr[kMaxRoundsPerStep], inv_safe[kMaxRoundsPerStep];
+    __shared__ float thr[kMaxRoundsPerStep], lim[kMaxRoundsPerStep], inv_safe[kMaxRoundsPerStep];
     __shared__ unsigned hist[256];
     __shared__ int cnt0, fill, mode, drop_safe;
     __shared__ unsigned need;
@@ -1659,8 +1687,10 @@ __device__ __forceinline__ void select_frame(const Pools &P) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const float t = fminf(before, m[u]);
+            const float err = filter_error(f, t);
             thr[4 * threadIdx.x + u] = t;
-            inv_safe[4 * threadIdx.x + u] = __frcp_rn(t * (1.0f / 32768.0f) + 0.5f);
+            lim[4 * threadIdx.x + u] = t + 4.0f * err;
+            inv_safe[4 * threadIdx.x + u] = __frcp_rn(2.0f * err);
         }
     }
     if (threadIdx.x == 0) {
@@ -1677,8 +1707,7 @@ __device__ __forceinline__ void select_frame(const Pools &P) {
     for (int j = threadIdx.x; j < nh; j += blockDim.x) {
         const int i = list ? list[j] : j;
         const float s = P.hS32[hb + i];
-        const float pm = thr[round_of(f, P.hId[hb + i])];
-        my += (s <= cand_limit(pm)) ? 1 : 0;
+        my += (s <= lim[round_of(f, P.hId[hb + i])]) ? 1 : 0;
     }
     my = warp_sum(my);
     if ((threadIdx.x & 31) == 0) atomicAdd(&cnt0, my);
@@ -1743,9 +1772,8 @@ __device__ __forceinline__ void select_frame(const Pools &P) {
                 const float s = P.hS32[hb + i];
                 const int64_t id = P.hId[hb + i];
                 const int r = round_of(f, id);
-                const float pm = thr[r];
-                if (!(s <= cand_limit(pm))) continue;
-                const unsigned long long key = cand_key(s, pm, inv_safe[r], id, f.step_first);
+                if (!(s <= lim[r])) continue;
+                const unsigned long long key = cand_key(s, thr[r], inv_safe[r], id, f.step_first);
                 if ((key & hi_mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
             }
             __syncthreads();
@@ -1770,10 +1798,9 @@ __device__ __forceinline__ void select_frame(const Pools &P) {
         const float s = P.hS32[hb + i];
         const int64_t id = P.hId[hb + i];
         const int r = round_of(f, id);
-        const float pm = thr[r];
-        if (!(s <= cand_limit(pm))) continue;
+        if (!(s <= lim[r])) continue;
         if (mode == 1) {
-            const unsigned long long key = cand_key(s, pm, inv_safe[r], id, f.step_first);
+            const unsigned long long key = cand_key(s, thr[r], inv_safe[r], id, f.step_first);
             if (key > kmax) {
                 if (__uint_as_float((unsigned)(key >> 32)) <= 1.0f) drop_safe = 1;
                 continue;
@@ -2671,9 +2698,8 @@ __device__ __forceinline__ void copy_block(const char *__restrict__ src, char *_
 
 // Small admissions in one launch: frames whose records, slots and points lie in
 // page-locked host memory, read over the link. A cluster of 8 CTAs per frame
-// copies the points, finds the box, normalises and packs them (k_prep_bounds and
-// k_prep_pack's work) and builds the PROSAC table; with `clear` the first CTA
-// zeroes the counters. Instead of a memset, four copies and four kernels: a call on 2000
+// copies the points, finds their centre, normalises and packs them (k_prep_pack's work)
+// and builds the PROSAC table; with `clear` the first CTA zeroes the counters. Instead of a memset, four copies and four kernels: a call on 2000
 // points 256 -> 221 us, on 301 points 223 -> 208, 24 frames with masks 1267 -> 955 us.
 constexpr int kAdmitCtas = 8, kAdmitThreads = 512;
 __global__ void __cluster_dims__(kAdmitCtas, 1, 1) __launch_bounds__(kAdmitThreads)
@@ -2682,14 +2708,9 @@ __global__ void __cluster_dims__(kAdmitCtas, 1, 1) __launch_bounds__(kAdmitThrea
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ FrameDev f;
-    __shared__ unsigned long long bmin[3], bmax[3];  // this CTA's points
     const int a = blockIdx.x / kAdmitCtas, rank = (int)cluster.block_rank();
     for (int i = threadIdx.x; i < (int)(sizeof(FrameDev) / 16); i += blockDim.x)
         reinterpret_cast<int4 *>(&f)[i] = reinterpret_cast<const int4 *>(recs + a)[i];
-    if (threadIdx.x < 3) {
-        bmin[threadIdx.x] = ~0ull;
-        bmax[threadIdx.x] = 0ull;
-    }
     const int slot = slots[a];
     const char *suv = src[2 * a], *sxyz = src[2 * a + 1];
     if (clear && blockIdx.x == 0 && threadIdx.x < kCNum) P.counters[threadIdx.x] = 0;
@@ -2703,42 +2724,12 @@ __global__ void __cluster_dims__(kAdmitCtas, 1, 1) __launch_bounds__(kAdmitThrea
         copy_block(suv + 16 * i0, (char *)(P.uv64 + 2 * (base + i0)), 16 * (n1 - i0));
         copy_block(sxyz + 24 * i0, (char *)(P.X64 + 3 * (base + i0)), 24 * (n1 - i0));
     }
-    __syncthreads();
-    double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
-    for (int64_t i = i0 + threadIdx.x; i < n1; i += blockDim.x) {
-        const double v[3] = {P.X64[3 * (base + i)], P.X64[3 * (base + i) + 1], P.X64[3 * (base + i) + 2]};
-        if (!(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]))) continue;  // staged as an outlier
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            lo[k] = fmin(lo[k], v[k]);
-            hi[k] = fmax(hi[k], v[k]);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[k] = fmin(lo[k], __shfl_down_sync(0xffffffffu, lo[k], o));
-            hi[k] = fmax(hi[k], __shfl_down_sync(0xffffffffu, hi[k], o));
-        }
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(&bmin[k], dbl_to_ordered(lo[k]));
-            atomicMax(&bmax[k], dbl_to_ordered(hi[k]));
-        }
-    }
-    cluster.sync();
-    unsigned long long bl[3] = {~0ull, ~0ull, ~0ull}, bh[3] = {0ull, 0ull, 0ull};
-    for (int r = 0; r < kAdmitCtas; ++r)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            bl[k] = min(bl[k], *cluster.map_shared_rank(&bmin[k], r));
-            bh[k] = max(bh[k], *cluster.map_shared_rank(&bmax[k], r));
-        }
+    cluster.sync();  // every CTA's points are in the pool
     double cc[3];
-    box_centre(bl, bh, cc);
+    frame_centre(P.X64 + 3 * base, f.n, cc);
     if (rank == 0) {
         if (threadIdx.x == 0)
-            for (int k = 0; k < 3; ++k) f.bmin[k] = bl[k], f.bmax[k] = bh[k], f.centre[k] = cc[k];
+            for (int k = 0; k < 3; ++k) f.centre[k] = cc[k];
         __syncthreads();
         for (int i = threadIdx.x; i < (int)(sizeof(FrameDev) / 16); i += blockDim.x)
             reinterpret_cast<int4 *>(P.frames + slot)[i] = reinterpret_cast<const int4 *>(&f)[i];
@@ -2746,7 +2737,6 @@ __global__ void __cluster_dims__(kAdmitCtas, 1, 1) __launch_bounds__(kAdmitThrea
     const double itau = 1.0 / f.tau;
     for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) pack_point(P, f, base, i, cc, itau);
     if (rank == 0 && f.prosac) prosac_table(P, f);
-    cluster.sync();  // no CTA leaves while its box may be read
 }
 
 // The bundle-adjust form: one frame's points (and weights) straight into the LM
