@@ -2209,47 +2209,44 @@ constexpr int kLMCluster = 8;  // CTAs cooperating on one frame's LM
 constexpr int kLMSums = 28;  // 21 J^T W J, 6 J^T W r, cost
 enum LMLoss : int32_t { kLossCauchy = 0, kLossTruncated = 1, kLossHuber = 2, kLossTrivial = 3 };
 
-__device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
-
-// Two compensated FP32 sums (S - C, S the rounded sum, C its excess) added to two
-// others in place (packed FP32x2): the rounding error of S + S2 (Knuth's
-// TwoSum) goes into C.
-__device__ __forceinline__ void pair_add2(uint64_t &S, uint64_t &C, uint64_t S2, uint64_t C2) {
-    const uint64_t t = f2add_rn(S, S2), b = f2sub(t, S);
-    const uint64_t e = f2add_rn(f2sub(S, f2sub(t, b)), f2sub(S2, b));
-    C = f2sub(f2add_rn(C, C2), e);
-    S = t;
+// S - C of a compensated FP32 sum, in FP64. Only S is converted, at a quarter of the rate
+// of other instructions: C's bits, moved to a double's places as they are, make
+// C 2^-896 exactly (the exponents' biases differ by 896; denormals and 0 too), which
+// the subtraction scales back.
+__device__ __forceinline__ double compensated(float S, float C) {
+    const int b = __float_as_int(C);
+    return fma(__hiloint2double((b >> 3) & 0x8FFFFFFF, b << 29), -0x1p896, (double)S);
 }
 
-// Sum over the warp of 28 compensated FP32 sums per lane, in pairs: lane k returns
-// the sum of value k in FP64. Reduce-scatter by recursive halving: a lane trades the
-// half of its pairs that its partner keeps (8 + 4 + 2 + 1 pairs at distances 16, 8,
-// 4, 2), then one value of the last pair at distance 1. In FP32 pairs, since
-// converting 56 values a lane to FP64 first takes longer than the whole reduction.
-__device__ __forceinline__ double warp_scatter_pairs(const uint64_t (&S)[14], const uint64_t (&C)[14]) {
+// Sum over the warp of 28 compensated FP32 sums per lane (S - C, two to a register
+// pair), in FP64: lane k returns the sum of value k. Reduce-scatter by recursive
+// halving: a lane trades the half of its values that its partner keeps, 16, 8, 4, 2
+// and 1 of them. (Left in FP32 pairs down to the last exchange the sums keep 48 bits
+// instead of 53; an LM iteration on 2000 points takes 4.6 us that way, 4.8 this way,
+// 5.0 with C converted like S.)
+__device__ __forceinline__ double warp_scatter(const uint64_t (&S)[14], const uint64_t (&C)[14]) {
     const int lane = threadIdx.x & 31;
-    uint64_t s[16], c[16];
+    double a[32];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) s[k] = k < 14 ? S[k] : 0ull, c[k] = k < 14 ? C[k] : 0ull;
+    for (int k = 0; k < 16; ++k) {
+        float s0 = 0.0f, s1 = 0.0f, c0 = 0.0f, c1 = 0.0f;
+        if (k < 14) {
+            f2unpack(S[k], s0, s1);
+            f2unpack(C[k], c0, c1);
+        }
+        a[2 * k] = k < 14 ? compensated(s0, c0) : 0.0;
+        a[2 * k + 1] = k < 13 ? compensated(s1, c1) : 0.0;  // (the 28th is not used)
+    }
 #pragma unroll
-    for (int h = 8; h >= 1; h >>= 1) {
-        const bool upper = (lane & (2 * h)) != 0;
+    for (int h = 16; h >= 1; h >>= 1) {
+        const bool upper = (lane & h) != 0;
 #pragma unroll
         for (int k = 0; k < h; ++k) {
-            if (k + h >= 14 && k >= 14) continue;
-            const uint64_t gs = shfl_xor64(upper ? s[k] : s[k + h], 2 * h);
-            const uint64_t gc = shfl_xor64(upper ? c[k] : c[k + h], 2 * h);
-            s[k] = upper ? s[k + h] : s[k];
-            c[k] = upper ? c[k + h] : c[k];
-            pair_add2(s[k], c[k], gs, gc);
+            const double keep = upper ? a[k + h] : a[k], give = upper ? a[k] : a[k + h];
+            a[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
         }
     }
-    float s0, s1, c0, c1;
-    f2unpack(s[0], s0, s1);
-    f2unpack(c[0], c0, c1);
-    const bool odd = (lane & 1) != 0;
-    const float gs = __shfl_xor_sync(0xffffffffu, odd ? s0 : s1, 1), gc = __shfl_xor_sync(0xffffffffu, odd ? c0 : c1, 1);
-    return ((double)(odd ? s1 : s0) - (double)(odd ? c1 : c0)) + ((double)gs - (double)gc);
+    return a[0];
 }
 
 // What the LM evaluates: the camera and loss of a frame.
@@ -2279,9 +2276,8 @@ __device__ __forceinline__ void kahan_add2(uint64_t &S, uint64_t &C, uint64_t x)
 // few instructions on a short chain: the Cauchy cost, sum log(1 + a), a = r^2 /
 // s^2, is taken as one log1p a thread, of the product of the 1 + a kept as q =
 // product - 1 (exact to rounding for small a); the Kahan sums run two to a packed
-// instruction and stay FP32 pairs in the warp's reduction. What bounds it is the
-// latency of one point's FP64 and FP32 chain (about 1400 cycles, two points in
-// flight) and of the reduction (about 1300).
+// instruction. What bounds it is the latency of one point's FP64 and FP32 chain (about
+// 1400 cycles, two points in flight) and the warp's reduction (about 1700).
 template <bool kCauchy>
 __device__ __forceinline__ int lm_pass(const Pools &P, int64_t base, int i0, int i1, const double *pose,
                                        const float *Rf, const LMModel &m, double (*scratch)[kLMSums]) {
@@ -2402,7 +2398,7 @@ __device__ __forceinline__ int lm_pass(const Pools &P, int64_t base, int i0, int
     if (warp < nw) {
         // Lanes 0 to 26: the accumulators; the cost (any lane's) goes to place 27.
         const int lane = threadIdx.x & 31;
-        double s = warp_scatter_pairs(S, C);
+        double s = warp_scatter(S, C);
         if (kCauchy) cost += log1p(q);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
@@ -2459,8 +2455,8 @@ __device__ __forceinline__ void cholesky_solve6(const double *H, double lambda, 
 // accepts or rejects and solves for the next candidate, each for itself and all
 // alike, so an iteration costs one pass, two CTA barriers and, in a cluster,
 // one cluster barrier. Measured cycles an iteration (pass, sums, solve), before
-// -> now: 799 inliers on one CTA 12000 -> 9000 (6500 + 500 + 2000), 13986 on 8 CTAs
-// 26500 -> 15700 (12000 + 1800 + 1900); the LM of the 256-frame batch 0.9 -> 0.55 ms.
+// -> now: 799 inliers on one CTA 12000 -> 9400 (6900 + 500 + 2000), 13986 on 8 CTAs
+// 26500 -> 16300 (12600 + 1800 + 1900); the LM of the 256-frame batch 0.9 -> 0.58 ms.
 template <int CL>
 __device__ __forceinline__ void lm_frame(const Pools &P, int slot) {
     namespace cg = cooperative_groups;
