@@ -235,6 +235,8 @@ def config1_scoring(ctx, reps=5, hr=0):
     pairs = d["hypotheses"] * f.n
     return {"config": "scoring-bound frame: N=20000, 15 % inliers, exactly 4096 samples (early stop off)",
             "samples": d["samples"], "hypotheses": d["hypotheses"], "pairs": pairs,
+            "pairs_accounting": "every hypothesis on every point, as a one-pass scorer needs; two-pass scoring "
+                                "evaluates fewer; gpu_ms_per_call holds the points' transfer and preparation too",
             "gpu_ms_per_call": statistics.mean(ms), "pairs_per_s": pairs / (statistics.mean(ms) / 1000.0),
             "candidate_overflow": d["candidate_overflow"]}
 

@@ -134,7 +134,10 @@ typedef struct tbr_stats {
     int32_t lm_invalid_steps;
     double lm_initial_cost;
     double lm_cost;
-    double gpu_ms;                /* device time of the call (CUDA events) */
+    double gpu_ms;                /* device time of the call (CUDA events), from the points' preparation to the
+                                     refinement's end; copies of large host batches and of device arrays come
+                                     before it, small host calls read their points over the link inside it.
+                                     tbr_bundle_adjust: the refinement alone */
 } tbr_stats;
 
 typedef struct tbr_context tbr_context;

@@ -1252,7 +1252,8 @@ static tbr_status admit_host_frames(Engine &E, const std::vector<FrameHost> &fr,
 // kernel reads records and points from page-locked memory -- the staging buffer, or
 // the caller's own arrays where they are page-locked and large enough for the
 // query to cost less than the copy -- and does the whole preparation
-// (k_admit_points); with `clear` it also zeroes the counters.
+// (k_admit_points); with `clear` it also zeroes the counters. E.ev0 marks its start: the
+// preparation is device work of the call.
 constexpr size_t kMappedQueryBytes = 128u << 10;
 
 // Copies a frame's arrays into its staging place, or finds the caller's page-locked
@@ -1294,6 +1295,7 @@ static tbr_status admit_small(Engine &E, const std::vector<FrameHost> &fr, const
     std::vector<CopyJob> copies;
     for (size_t i = 0; i < n; ++i) stage_or_map(E, A, i, copies, src + 2 * i);
     parallel_copy(E.helpers, copies);
+    TBR_CUDA(cudaEventRecord(E.ev0, E.stream));
     k_admit_points<<<(int)n * kAdmitCtas, kAdmitThreads, 0, E.stream>>>(
         E.P, stage_alias(E, A.hd), stage_alias(E, A.ha), (const char *const *)stage_alias(E, src), E.d_active,
         clear ? 1 : 0);
@@ -1553,8 +1555,10 @@ static tbr_status enqueue_frames(Engine &E, const std::vector<FrameHost> &fr, co
         bool prepared = false;
         st = admit_frames(E, fr, o, slots, max_n, &prepared, &devs, device_points, true);
         if (st == TBR_OK) {
-            TBR_CUDA(cudaEventRecord(E.ev0, E.stream));
-            if (!prepared) E.launch_prep((int)slots.size(), max_n);
+            if (!prepared) {
+                TBR_CUDA(cudaEventRecord(E.ev0, E.stream));
+                E.launch_prep((int)slots.size(), max_n);
+            }
             E.pp = o.pp;
             st = E.launch_graph((int)slots.size(), o.hr);
         }
