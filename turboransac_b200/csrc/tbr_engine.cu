@@ -1248,13 +1248,21 @@ static tbr_status admit_host_frames(Engine &E, const std::vector<FrameHost> &fr,
     return st;
 }
 
-// Small host admissions (one frame, or frames below kZeroCopyMinBytes together): one
-// kernel reads records and points from page-locked memory -- the staging buffer, or
-// the caller's own arrays where they are page-locked and large enough for the
-// query to cost less than the copy -- and does the whole preparation
+// Small host admissions (frames below kZeroCopyMinBytes together, one frame below
+// kOneFrameIngestBytes): one kernel reads records and points from page-locked memory --
+// the staging buffer, or the caller's own arrays where they are page-locked and large
+// enough for the query to cost less than the copy -- and does the whole preparation
 // (k_admit_points); with `clear` it also zeroes the counters. E.ev0 marks its start: the
 // preparation is device work of the call.
+//
+// One frame's kernel reads the link with 8 CTAs, 27 GB/s, and prepares with them;
+// ingestion reads 51 GB/s and prepares with 64, after 30 us more of launches and, for
+// pageable arrays, of waiting for the helpers. A call with 64 samples, no refinement,
+// by this kernel / by ingestion: pageable arrays of 200000 points 1.10 / 1.26 ms, 500000
+// 2.07 / 1.87, 1000000 3.87 / 3.37, 4000000 15.2 / 13.9; page-locked 200000 0.62 / 0.52,
+// 1000000 2.75 / 2.28, 4000000 11.6 / 9.9.
 constexpr size_t kMappedQueryBytes = 128u << 10;
+constexpr size_t kOneFrameIngestBytes = 16u << 20;
 
 // Copies a frame's arrays into its staging place, or finds the caller's page-locked
 // ones; src: their two addresses as the device sees them.
@@ -1306,9 +1314,9 @@ static tbr_status admit_small(Engine &E, const std::vector<FrameHost> &fr, const
 
 // Both halves through the context's own staging buffer. With device_points the
 // frames' point arrays are device memory of this GPU: they are copied into the
-// pool by one kernel, with no host staging. Multi-frame host batches of some
-// size are ingested zero-copy (admit_host_frames), smaller ones and single frames by
-// admit_small, which also prepares them (*prepared).
+// pool by one kernel, with no host staging. Large host frames (kZeroCopyMinBytes
+// together, kOneFrameIngestBytes alone) are ingested zero-copy (admit_host_frames),
+// smaller ones admitted by admit_small, which also prepares them (*prepared).
 static tbr_status admit_frames(Engine &E, const std::vector<FrameHost> &fr, const RunOptions &o,
                                std::vector<int> &slots, int64_t &max_n, bool *prepared,
                                std::vector<FrameDev> *host_devs = nullptr, bool device_points = false,
@@ -1316,9 +1324,9 @@ static tbr_status admit_frames(Engine &E, const std::vector<FrameHost> &fr, cons
     *prepared = false;
     size_t in_bytes = 0;
     for (auto &f : fr) in_bytes += 40 * (size_t)f.n;
-    const bool small = !device_points && (fr.size() < 2 || in_bytes < kZeroCopyMinBytes);
+    const bool small = !device_points && in_bytes < (fr.size() < 2 ? kOneFrameIngestBytes : kZeroCopyMinBytes);
     if (clear && !small) TBR_CUDA(cudaMemsetAsync(E.P.counters, 0, 8 * kCNum, E.stream));
-    if (!device_points && fr.size() >= 2 && in_bytes >= kZeroCopyMinBytes) {
+    if (!device_points && !small) {
         std::vector<FrameDev> d;
         tbr_status st = admit_host_frames(E, fr, o, slots, max_n, d, false);
         if (host_devs) *host_devs = d;
@@ -2980,6 +2988,7 @@ tbr_status tbr_debug_score_samples(tbr_context *ctx, const double *points2D, con
     bool prepared = false;
     tbr_status st = admit_frames(E, {fh}, o, slots, max_n, &prepared, nullptr, false, true);
     if (st) return st;
+    if (!prepared) E.launch_prep(1, max_n);
     E.P.prune = 0;  // every hypothesis's score is wanted
     k_plan<<<1, kMaxActive, 0, E.stream>>>(E.P);
     k_sample_p3p<<<E.p3p_grid, 128, 0, E.stream>>>(E.P);
