@@ -802,9 +802,9 @@ def main():
             "candidate_overflow_frames": int(sum(int(r["candidate_overflow"]) for r in res)),
             "serving": serving,
             "speedup_vs_plain": (value / plain["frames_per_s"]) if plain else None,
-            # per graph launch: the reset, per engine step 8 RANSAC kernels + 3
-            # refinement kernels + the loop test, and the last step's refinement
-            "gpu_launches": args.steps * (1 + 12 * steps_per_run + 3),
+            # per graph launch: the reset, per engine step 7 kernels (9 where steps
+            # may score in two passes), and the refinement's 3
+            "gpu_launches": args.steps * (1 + (9 if prof["k_prune"][1] else 7) * steps_per_run + 3),
             "clocks": clocks,
         }
         print(json.dumps(line), flush=True)

@@ -352,16 +352,6 @@ __device__ __forceinline__ void p3p_finish(const P3PCtx &c, double d0, double d1
     pose_from_depths(c.x, c.X0, d0, d1, d2, c.Mi, P);
 }
 
-// P3P for three unit bearings and world points; up to 4 poses written to
-// out[12*k]; returns their number (p3p.cuh:9-222).
-__device__ __forceinline__ int p3p_solve(const d3 xin[3], const d3 Xin[3], double *out) {
-    P3PCtx c;
-    double dep[12];
-    const int n = p3p_candidates(xin, Xin, c, dep);
-    for (int k = 0; k < n; ++k) p3p_finish(c, dep[3 * k], dep[3 * k + 1], dep[3 * k + 2], out + 12 * k);
-    return n;
-}
-
 // ---------------------------------------------------------- quaternions -----
 // R (row-major) -> unit quaternion (w, x, y, z), Shepperd branches then
 // normalisation (pose_utils.cuh:13-58).

@@ -245,8 +245,12 @@ struct CopyJob {
     const void *src;
     size_t bytes;
 };
-// From kCopyParallel bytes on with the helpers (they take about 30 us to wake; this
-// thread copies meanwhile), in pieces taken in turn.
+// From kCopyParallel bytes on with the helpers, in pieces taken in turn (they take about
+// 30 us to wake, more after a pause; this thread copies meanwhile). Masks of poses on
+// arrays that are in no cache, one call after another: 12000 points (480 KB, no
+// helpers) 73 us, 14000 57, 20000 63, 50000 105; with 2 ms between the calls 79, 100,
+// 109 and 180; by copies of one thread, upload, kernel and download 92, 99, 125 and 258,
+// or 99, 108, 132 and 265.
 constexpr size_t kCopyParallel = 512u << 10, kCopyPiece = 64u << 10;
 static void parallel_copy(HelperThreads &helpers, const std::vector<CopyJob> &jobs) {
     size_t total = 0;
@@ -654,7 +658,7 @@ class Engine {
             beg(5); launch_prune(Q, n_active, st); end(5);
             beg(10); launch_score(Q, hr, pp, st, 1); end(10);
         }
-        beg(4); k_select<<<n_active, 1024, 0, st>>>(Q); end(4);  // a frame's ~4000 hypotheses: 1024 threads (6.51 ms a batch, 256: 6.59)
+        beg(4); k_select<<<n_active, 1024, 0, st>>>(Q); end(4);  // (256 threads a frame: 1 % more a batch, when a batch took 6.5 ms)
         beg(6); k_rescore<<<rescore_grid, 256, 0, st>>>(Q); end(6);
         beg(7);
         if (loop) k_finalize_loop<<<n_active, 256, 0, st>>>(Q, *loop, 100000ull);

@@ -566,10 +566,10 @@ __global__ void k_plan(Pools P) {
 // root filters); the warp then shares out the candidates -- 0 to 4 a sample --
 // so that the depth polish and the pose, most of the arithmetic, run on full
 // warps instead of once per candidate slot that any lane of the warp needs.
-// Every candidate runs p3p_solve's own steps (p3p_finish) and keeps its order
-// (hId = sample * 4 + solution); the compiler may fuse a multiply-add
-// differently than in a per-thread loop, so poses can differ from that form in
-// the last bits, never in which samples give solutions.
+// Every candidate keeps its order (hId = sample * 4 + solution) and its steps
+// (p3p_finish); the compiler may fuse a multiply-add differently than in a
+// per-thread loop, so poses can differ from that form in the last bits, never in
+// which samples give solutions.
 // What bounds it is the latency of one sample's FP64 chain (16 warps an SM, the
 // FP64 pipe a fifth busy) and, with many samples, the stores of the poses, 96 and 48
 // bytes a candidate, in 16-byte words since each lane's lie apart. Both lines of the
@@ -2302,20 +2302,10 @@ __device__ __forceinline__ int lm_pass(const Pools &P, int64_t base, int i0, int
         const double Z1 = R[3] * X0d + R[4] * X1d + R[5] * X2d + t[1];
         const double Z2 = R[6] * X0d + R[7] * X1d + R[8] * X2d + t[2];
         const bool valid = Z2 >= 0.0;
-        double inv_z, r0, r1, r_squared;
-        double lc = 0.0, a = 0.0;
-        if (kCauchy) {
-            inv_z = 1.0 / Z2;
-            r0 = (m.fx * (Z0 * inv_z) + m.cx) - u;
-            r1 = (m.fy * (Z1 * inv_z) + m.cy) - v;
-            r_squared = r0 * r0 + r1 * r1;
-            a = r_squared * m.inv_sq;
-        } else {
-            inv_z = 1.0 / Z2;
-            r0 = (m.fx * (Z0 * inv_z) + m.cx) - u;
-            r1 = (m.fy * (Z1 * inv_z) + m.cy) - v;
-            r_squared = r0 * r0 + r1 * r1;
-        }
+        const double inv_z = 1.0 / Z2;
+        const double r0 = (m.fx * (Z0 * inv_z) + m.cx) - u, r1 = (m.fy * (Z1 * inv_z) + m.cy) - v;
+        const double r_squared = r0 * r0 + r1 * r1;
+        double lc = 0.0, a = kCauchy ? r_squared * m.inv_sq : 0.0;
         // FP32 Jacobian from the FP64 projection and residual.
         const float iz = (float)inv_z, z0 = (float)(Z0 * inv_z), z1 = (float)(Z1 * inv_z);
         const float rx = (float)r0, ry = (float)r1;
